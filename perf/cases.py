@@ -148,27 +148,41 @@ class _Shape:
         self.moe_intermediate_size, self.hidden_size = case["width"], case["dims"]
 
 
-def _prepare_layer(case: dict, g, x: torch.Tensor) -> dict:
+def _layer_tensors(case: dict, g, x: torch.Tensor) -> tuple:
+    """(gate, up, down, router rows) of an affine layer; sets x's first input when the case is skewed."""
+
     count = case["experts"] + (1 if case["shared"] else 0)
     dims, width, dtype = case["dims"], case["width"], SCALES[case["scales"]]
     gate, up = (_affine_matrix(g, count, width, dims, dtype) for _ in range(2))
     down = _affine_matrix(g, count, dims, width, dtype)
-    layer = moe.Routed(_router(case, g, x), experts.make([gate, up], down, 64), case["top_k"], case["shared"])
+    return gate, up, down, _router(case, g, x)
+
+
+def _prepare_layer(case: dict, g, x: torch.Tensor) -> dict:
+    gate, up, down, router = _layer_tensors(case, g, x)
+    layer = moe.Routed(router, experts.make([gate, up], down, 64), case["top_k"], case["shared"])
     if case["form"] == "runner":
         return {"case": case, "x": x, "runner": moe.Runner(layer, case["rows"])}
     return {"case": case, "x": x, "layer": layer}
 
 
-def _prepare_exl3(case: dict, g, x: torch.Tensor) -> dict:
-    dims, width, rows = case["dims"], case["width"], case["rows"]
+def _exl3_tensors(case: dict, g) -> list:
+    """[gate, up, down], each a list over the experts of (trellis, suh, svh)."""
+
+    dims, width = case["dims"], case["width"]
     # a width a tensor, the same for every seed (as a checkpoint's): 2 to 8 bits
     widths = np.random.RandomState(5).randint(2, 9, (case["experts"], 3))
 
     def bits(e: int, m: int) -> int:
         return case["bits"] or int(widths[e, m])
 
-    gate, up, down = ([_exl3_matrix(g, *kn, bits(e, m)) for e in range(case["experts"])]
-                      for m, kn in enumerate([(dims, width), (dims, width), (width, dims)]))
+    return [[_exl3_matrix(g, *kn, bits(e, m)) for e in range(case["experts"])]
+            for m, kn in enumerate([(dims, width), (dims, width), (width, dims)])]
+
+
+def _prepare_exl3(case: dict, g, x: torch.Tensor) -> dict:
+    dims, rows = case["dims"], case["rows"]
+    gate, up, down = _exl3_tensors(case, g)
     ex = exl3.prepare(gate, up, down, case["codebook"], device=DEV)
     s = {"case": case, "x": x, "router": _router(case, g, x), "experts": ex,
          "buf": moe.MoEBuffers(rows, _Shape(case), DEV, shared=False),
@@ -194,9 +208,13 @@ def _exl3_step(s: dict, x: torch.Tensor) -> None:
     exl3.routed(x, buf.pick, buf.wts, s["experts"], s["scratch"], s["out"], case["rows"])
 
 
-def prepare(case: dict, seed: int) -> dict:
+def _tokens(case: dict, seed: int) -> tuple:
     g = torch.Generator(device=DEV).manual_seed(seed)
-    x = torch.randn((case["rows"], case.get("dims") or case["k"]), generator=g, device=DEV).to(torch.bfloat16)
+    return g, torch.randn((case["rows"], case.get("dims") or case["k"]), generator=g, device=DEV).to(torch.bfloat16)
+
+
+def prepare(case: dict, seed: int) -> dict:
+    g, x = _tokens(case, seed)
     if case["kind"] == "layer":
         return _prepare_layer(case, g, x)
     if case["kind"] == "exl3":
@@ -228,6 +246,106 @@ def run(state: dict):
     if case["prompt"]:
         return exl3_prefill.matmul(state["linear"], x, state["out"], state["ws"])
     return state["linear"](x)
+
+
+# ---- the same results in 64 bits, by plain torch ---------------------------------------------------------------------
+
+
+def _affine_weight(words: torch.Tensor, scales: torch.Tensor, biases: torch.Tensor) -> torch.Tensor:
+    """[N, K] in 64 bits: nibble i of a word is input i, groups of 64 inputs share a scale and a bias."""
+
+    q = (words.unsqueeze(-1) >> (4 * torch.arange(8, device=DEV))) & 15
+    q = q.reshape(words.shape[0], -1, 64).double()
+    return (q * scales.double().unsqueeze(-1) + biases.double().unsqueeze(-1)).reshape(words.shape[0], -1)
+
+
+def _codebook(name: str) -> torch.Tensor:
+    """The 16-bit values of the 65536 states, as doubles."""
+
+    s = np.arange(65536, dtype=np.uint64)
+    if name == "mul1":
+        v = (s * 0x83DCD12D) & 0xFFFFFFFF
+        total = 1024.0 + sum(((v >> k) & 255).astype(np.float64) for k in (0, 8, 16, 24))
+        scale, bias = np.array([0x1EEE, 0xC931], np.uint16).view(np.float16).astype(np.float64)
+        return torch.from_numpy((total * scale + bias).astype(np.float16).astype(np.float64)).to(DEV)
+    v = (s * 0xCBAC1FED if name == "mcg" else s * 89226354 + 64248484) & 0xFFFFFFFF
+    v = (v & 0x8FFF8FFF) ^ 0x3B603B60
+    low, high = ((v >> k).astype(np.uint16).view(np.float16) for k in (0, 16))
+    return torch.from_numpy((low + high).astype(np.float64)).to(DEV)
+
+
+def _trellis_weight(trellis: torch.Tensor, book: torch.Tensor) -> torch.Tensor:
+    """[K, N] in 64 bits.  A 16 x 16 tile is a circular stream of its 32-bit words, first bit first; value p's state
+    is the 16 bits that end where the widths of the values up to p end."""
+
+    k2 = trellis.shape[-1] // 8
+    words = trellis.view(torch.int32).long() & 0xFFFFFFFF
+    p = torch.arange(256, device=DEV)
+    first = (p >> 1) * k2 + torch.where(p % 2 == 1, k2, k2 >> 1) - 16 + 128 * k2
+    at, off = (first // 32) % (4 * k2), first % 32
+    # the 16 bits from bit ``off`` of a word and, where it ends, of the next
+    state = ((words[..., at] << off) & 0xFFFFFFFF | (words[..., (at + 1) % (4 * k2)] << off >> 32)) >> 16
+    lane, j = p // 8, p % 8
+    row, col = 2 * (lane % 4) + (j & 1) + 8 * ((j >> 1) & 1), lane // 4 + 8 * (j >> 2)
+    tiles = torch.empty((*words.shape[:2], 16, 16), dtype=torch.float64, device=DEV)
+    tiles[:, :, row, col] = book[state]
+    return tiles.transpose(1, 2).reshape(16 * words.shape[0], 16 * words.shape[1])
+
+
+def _rotated(x: torch.Tensor) -> torch.Tensor:
+    i = torch.arange(128, device=DEV)
+    bits = sum(((i[:, None] & i[None, :]) >> k) & 1 for k in range(7))
+    return (x.reshape(-1, x.shape[1] // 128, 128) @ ((1 - 2 * (bits % 2)).double() / math.sqrt(128))).reshape(x.shape)
+
+
+def _exl3_product(x: torch.Tensor, matrix: tuple, book: torch.Tensor) -> torch.Tensor:
+    trellis, suh, svh = matrix
+    return _rotated(_rotated(x * suh.double()) @ _trellis_weight(trellis, book)) * svh.double()
+
+
+def _weighted(case: dict, x: torch.Tensor, router: torch.Tensor, expert) -> torch.Tensor:
+    """The layer's result [R, D]; ``expert(e, rows)`` gives expert e's rows."""
+
+    count = case["experts"]
+    logits = x @ router.double().T
+    best, pick = logits[:, :count].topk(case["top_k"], dim=1)
+    wts = torch.softmax(best, dim=1)
+    out = torch.zeros_like(x)
+    for e in range(count):
+        r, slot = (pick == e).nonzero(as_tuple=True)
+        if r.numel():
+            out.index_add_(0, r, wts[r, slot].unsqueeze(1) * expert(e, x[r]))
+    if case.get("shared"):
+        out += torch.sigmoid(logits[:, count:]) * expert(count, x)
+    return out
+
+
+def exact(case: dict, seed: int):
+    """``run``'s results for these inputs in 64 bits (the picks are whole numbers: no such value)."""
+
+    g, x16 = _tokens(case, seed)
+    if case["kind"] == "layer":
+        gate, up, down, router = _layer_tensors(case, g, x16)
+
+        def affine(e: int, rows: torch.Tensor) -> torch.Tensor:
+            a, b, c = (_affine_weight(*(t[e] for t in m)) for m in (gate, up, down))
+            return torch.nn.functional.silu(rows @ a.T) * (rows @ b.T) @ c.T
+
+        return _weighted(case, x16.double(), router, affine)
+    if case["kind"] == "exl3":
+        mats, book = _exl3_tensors(case, g), _codebook(case["codebook"])
+        router = _router(case, g, x16)
+
+        def trellis(e: int, rows: torch.Tensor) -> torch.Tensor:
+            act = torch.nn.functional.silu(_exl3_product(rows, mats[0][e], book)) * _exl3_product(rows, mats[1][e], book)
+            return _exl3_product(act, mats[2][e], book)
+
+        return {"out": _weighted(case, x16.double(), router, trellis), "pick": None}
+    n, k = case["n"], case["k"]
+    if case["kind"] == "affine":
+        w = _affine_matrix(g, 1, n, k, SCALES[case["scales"]])
+        return x16.double() @ _affine_weight(*(t[0] for t in w)).T
+    return _exl3_product(x16.double(), _exl3_matrix(g, k, n, case["bits"]), _codebook(case["codebook"]))
 
 
 # ---- what a pass cannot do without --------------------------------------------------------------------------------
