@@ -120,14 +120,18 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(bar)) : "memory");
 }
 
+// One try: the thread sleeps in hardware until the phase completes or `MBAR_NAP_NS` pass.  Without the time operand the
+// hardware gives up after a few cycles, and warps that wait for a pipeline stage then spin: in the prompt kernel and
+// the trellis kernel the waiting warps' loops took a third of all issue slots from the warps that decode.
+constexpr uint32_t MBAR_NAP_NS = 20000;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n.reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
       "selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
+      : "r"(smem_addr(bar)), "r"(parity), "r"(MBAR_NAP_NS)
       : "memory");
   return ok != 0;
 }
@@ -155,7 +159,7 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, ui
   uint64_t start = 0;
   for (uint32_t spin = 0; spin < (1u << 30); ++spin) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 1023u) == 1023u) {
+    if ((spin & 15u) == 15u) {
       const uint64_t now = global_ns();
       if (start == 0) start = now;
       else if (now - start > limit_ns) break;
@@ -171,10 +175,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// The slow path of mbar_wait_warp, out of line: inlined at every wait its loops cost registers and instruction cache.
+static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity); }
+
+// Arrives when `on`: a predicated instruction, no branch.
+__device__ __forceinline__ void mbar_arrive_if(uint64_t* bar, bool on) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, 0;\n@p mbarrier.arrive.shared::cta.b64 _, [%0];\n}\n" ::"r"(smem_addr(bar)),
+               "r"((uint32_t)on)
+               : "memory");
+}
+
 // The same for a whole warp (every lane calls it): one answer for all lanes, so the branch on it never splits a warp
 // in front of a warp-wide instruction.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;    // nearly always
+  return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity));
 }
 
 // global -> shared bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned), completion on `bar`

@@ -1,17 +1,26 @@
 // Prefill form of the grouped 4-bit experts: a grouped GEMM on the tcgen05 tensor cores.
 //
-// A CTA owns one unit = (plan item of <= 192 pairs, 128 output columns).  The roles are swapped against the usual
-// GEMM: the WEIGHTS are the MMA's A operand (M = 128 columns), the item's PAIRS the B operand (N = pairs rounded up to
-// 16, <= 192), so an expert with 140 pairs costs 144 / 128 of a full tile instead of two, and every weight is
-// dequantised exactly once.  Per group of 64 inputs (one pipeline stage):
-//   warp 13 (a lane)   bulk-copies the packed blocks (4 column blocks x M matrices) into a deep staging ring;
+// A CTA owns one unit = (plan item of <= 192 pairs, 128 weight rows).  The roles are swapped against the usual GEMM:
+// the WEIGHTS are the MMA's A operand (M = 128 rows: 128 output columns of one matrix, or 64 columns of gate and the
+// same 64 of up), the item's PAIRS the B operand (N = pairs rounded up to 16, <= 192), so an expert with 140 pairs
+// costs 144 / 128 of a full tile instead of two.  Per group of 64 inputs (one pipeline stage):
+//   warp 13 (a lane)   bulk-copies the packed blocks into a deep staging ring;
 //   warps 8-11         gather the pairs' input rows with 16-byte cp.async into the 128-byte-swizzled B tile;
 //   warps 0-7          turn nibbles into the prefill form's bf16 weights (w = bf16(q * s + b), one rounding) and
-//                      store them as the K-major, 128-byte-swizzled A tiles;
-//   warp 12 (a lane)   issues tcgen05.mma (cta_group::1, kind::f16, M = 128, K = 16) into fp32 accumulators in tensor
-//                      memory (gate at column 0, up at column 256), and commits each stage back to the producer.
+//                      store them straight into TENSOR MEMORY, a weight row a lane (tcgen05.st): two sets of four
+//                      warps take the even and the odd stages, each set with an A stage of its own;
+//   warp 12 (a lane)   issues tcgen05.mma (cta_group::1, kind::f16, M = 128, K = 16; A from tensor memory, B from
+//                      shared memory) into fp32 accumulators in tensor memory, and commits each stage back.
 // After the last group warps 0-11 read the accumulators (tcgen05.ld), apply the epilogue and store rows by pair id.
 // One fp32 chain over K in group order: a pair's bits do not depend on its item, its chunk or the call.
+//
+// What bounds it: shared-memory bandwidth and tensor issue, about even.  With the A tiles in shared memory a stage of
+// gate/up moved 154 KB through it at 192 pairs (of it 64 KB A written and read) and the K loop ran at 0.91 us a stage;
+// without them and with two CTAs an SM (256 of the 512 tensor-memory columns each: 192 of accumulators, two A stages
+// of 32; under 113 KB of shared memory) one unit's start, epilogue and waits run under the other's K loop.
+// A B200 at 2048 tokens of 128 experts (2048 x 768, top 8): gate/up 220 -> 177 us, down 182 -> 116 us; at 317 tokens with
+// a shared expert 172 -> 124 and 143 -> 77 us.  What is left is instruction issue (two thirds of the slots, the ALU pipe
+// 60 % busy): about 1000 of the dequantising warps' instructions a stage against 256 cycles of MMA.
 // (Replaces src/tensorfold/cuda/experts_prefill.cu:31-195: prefill_kernel and its launch.)
 
 #include "api.h"
@@ -19,32 +28,34 @@
 
 namespace tfb {
 
-constexpr int PF_COLS = 128;            // output columns a unit (MMA M)
+constexpr int PF_ROWS = 128;            // weight rows a unit (MMA M)
 constexpr int PF_MAXP = 192;            // pairs an item may hold (MMA N)
-constexpr int PF_CB = PF_COLS / COLS;   // packed column blocks a unit
-constexpr int PF_DQ_WARPS = 8;          // warps 0-7: dequantise, then the epilogue
+constexpr int PF_DQ_WARPS = 8;          // warps 0-7: dequantise (two sets of four), then the epilogue
 constexpr int PF_GA_WARPS = 4;          // warps 8-11: gather the pairs' input rows
 constexpr int PF_MMA_WARP = 12, PF_COPY_WARP = 13;
 constexpr int PF_THREADS = 14 * 32;
 constexpr int PF_GA_PER_THREAD = PF_MAXP * 8 / (PF_GA_WARPS * 32);   // 16-byte chunks a gather thread a stage
+constexpr int PF_TMEM_COLS = 256;       // a CTA's share of the tensor memory
+constexpr int PF_A_COL = PF_MAXP;       // its A stages: 2 x 32 columns behind the accumulators
 
-// Two rings: operand tiles (A per matrix and B) with SA stages, and the packed blocks as they come from HBM with SP
-// stages (deeper: it hides the HBM latency, and a stage is free again as soon as it has been dequantised).
 template <int M>
+constexpr int PF_CB = PF_ROWS / COLS / M;   // packed column blocks a unit
+
+// Two rings in shared memory: the B tiles (whole tiles of the item's own height, so items of fewer pairs get more
+// stages) and the packed blocks as they come from HBM.
 struct PrefillSmem {
-  static constexpr int SA = M == 2 ? 3 : 4;
-  static constexpr int SP = M == 2 ? 6 : 8;
-  static constexpr int A_BYTES = PF_COLS * 128;                 // one matrix: 128 rows of 64 bf16
-  static constexpr int B_BYTES = PF_MAXP * 128;
-  static constexpr int AB_BYTES = M * A_BYTES + B_BYTES;        // a multiple of 1024
-  static constexpr int PACKED_BYTES = PF_CB * M * BLOCK_BYTES;
-  static constexpr int PACKED_OFFSET = SA * AB_BYTES;
+  static constexpr int SP = 8;
+  static constexpr int B_BYTES = 3 * PF_MAXP * 128;
+  static constexpr int SB_MAX = 6;
+  static constexpr int PACKED_BYTES = PF_ROWS / COLS * BLOCK_BYTES;
+  static constexpr int PACKED_OFFSET = B_BYTES;
   static constexpr int TABLE_OFFSET = PACKED_OFFSET + SP * PACKED_BYTES;   // int out_row[PF_MAXP]
   static constexpr int BAR_OFFSET = (TABLE_OFFSET + PF_MAXP * 4 + 15) / 16 * 16;
-  static constexpr int NBARS = 2 * SP + 3 * SA + 1;
+  static constexpr int NBARS = 2 * SP + 2 * 2 + 2 * SB_MAX + 1;
   static constexpr int TMEM_OFFSET = BAR_OFFSET + NBARS * 8;
   static constexpr int TOTAL = TMEM_OFFSET + 16 + 1024;         // + slack to align the tiles to 1024 bytes
 };
+static_assert(2 * (PrefillSmem::TOTAL + 1024) <= 228 * 1024, "two CTAs share an SM");
 
 // ---- tcgen05 wrappers ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
@@ -72,13 +83,14 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
 }
 // kind::f16: D fp32, A and B bf16, both K-major, M = 128, N = n
 __device__ __forceinline__ uint32_t umma_idesc(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(PF_COLS >> 4) << 24);
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
 }
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+// A from tensor memory: lane = row, a 32-bit column = two consecutive inputs (K = 16: eight columns)
+__device__ __forceinline__ void umma_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accum)
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -93,6 +105,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16};\n" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -116,44 +137,52 @@ __device__ __forceinline__ uint32_t prefill_pair(uint32_t v, uint32_t sb) {
     return *reinterpret_cast<uint32_t*>(&r);
   } else {
     const float2 f = sb_pair<SB>(sb);
-    const float w0 = fmaf(f.x, bf16_lo(v) - 128.f, f.y), w1 = fmaf(f.x, bf16_hi(v) - 128.f, f.y);
-    __nv_bfloat162 r = __floats2bfloat162_rn(w0, w1);
+    const uint32_t k128 = BF16_128;
+    const __nv_bfloat162 q = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v),
+                                     *reinterpret_cast<const __nv_bfloat162*>(&k128));   // exact
+    const uint32_t qv = *reinterpret_cast<const uint32_t*>(&q);
+    const float2 w = ffma2(make_float2(bf16_lo(qv), bf16_hi(qv)), make_float2(f.x, f.x), make_float2(f.y, f.y));
+    __nv_bfloat162 r = __floats2bfloat162_rn(w.x, w.y);
     return *reinterpret_cast<uint32_t*>(&r);
   }
 }
 
 template <int M, int EPI, int SB>
-__global__ void __launch_bounds__(PF_THREADS, 1)
+__global__ void __launch_bounds__(PF_THREADS, 2)
 prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots, const uint8_t* __restrict__ W, int KG,
                int NB, const int* __restrict__ items, const int* __restrict__ counts, const int* __restrict__ members,
                void* __restrict__ out, int N, float limit) {
-  using SM = PrefillSmem<M>;
-  constexpr int SA = SM::SA, SP = SM::SP;
+  using SM = PrefillSmem;
+  constexpr int SP = SM::SP, CB = PF_CB<M>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   int* out_row = reinterpret_cast<int*>(smem + SM::TABLE_OFFSET);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::BAR_OFFSET);
   uint64_t* packed_full = bars;                  // [SP] the bulk copy landed
-  uint64_t* packed_free = bars + SP;             // [SP] the eight dequantising warps have read it
-  uint64_t* a_ready = bars + 2 * SP;             // [SA] the eight dequantising warps wrote their tiles
-  uint64_t* b_ready = a_ready + SA;              // [SA] the pairs' input rows landed
-  uint64_t* ab_free = b_ready + SA;              // [SA] the MMAs that read the stage retired
-  uint64_t* acc_ready = ab_free + SA;
+  uint64_t* packed_free = bars + SP;             // [SP] the four warps of the stage's set have read it
+  uint64_t* a_ready = bars + 2 * SP;             // [2] the four warps of the set stored their rows of the A stage
+  uint64_t* a_free = a_ready + 2;                // [2] the MMAs that read the A stage retired
+  uint64_t* b_ready = a_free + 2;                // [SB_MAX] the pairs' input rows landed
+  uint64_t* b_free = b_ready + SM::SB_MAX;       // [SB_MAX] the MMAs that read the B stage retired
+  uint64_t* acc_ready = b_free + SM::SB_MAX;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::TMEM_OFFSET);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nct = (NB + PF_CB - 1) / PF_CB;
+  const int nct = (NB + CB - 1) / CB;
   const int it = blockIdx.x / nct, ct = blockIdx.x - it * nct;
 
   if (tid == 0) {
     for (int s = 0; s < SP; ++s) {
       mbar_init(packed_full + s, 1);
-      mbar_init(packed_free + s, PF_DQ_WARPS);
+      mbar_init(packed_free + s, PF_DQ_WARPS / 2);
     }
-    for (int s = 0; s < SA; ++s) {
-      mbar_init(a_ready + s, PF_DQ_WARPS);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(a_ready + s, PF_DQ_WARPS / 2);
+      mbar_init(a_free + s, 1);
+    }
+    for (int s = 0; s < SM::SB_MAX; ++s) {
       mbar_init(b_ready + s, PF_GA_WARPS * 32);
-      mbar_init(ab_free + s, 1);
+      mbar_init(b_free + s, 1);
     }
     mbar_init(acc_ready, 1);
     mbar_fence_init();
@@ -162,8 +191,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
   pdl_wait();
   after_wait(X, items, counts, members);
   const bool live = it < ld_dep(counts);          // uniform over the CTA
-  constexpr uint32_t TMEM_COLS = 512;
-  if (live && warp == PF_MMA_WARP) tmem_alloc(tmem_slot, TMEM_COLS);
+  if (live && warp == PF_MMA_WARP) tmem_alloc(tmem_slot, PF_TMEM_COLS);
   int e = 0, first = 0, cnt = 0;
   if (live) {
     e = ld_dep(items + 3 * it);
@@ -177,43 +205,49 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
   if (!live) return;
   const uint32_t tmem_base = *tmem_slot;
   const int nmma = max(16, (cnt + 15) & ~15);
-  const int cb0 = ct * PF_CB, ncb = min(PF_CB, NB - cb0);        // packed column blocks of this unit
+  const int sb = min(SM::SB_MAX, SM::B_BYTES / (nmma * 128));    // B stages: 3 (192 pairs) to 6
+  const int b_bytes = nmma * 128;                                // a multiple of 1024: 8-row swizzle groups stay aligned
+  const int cb0 = ct * CB, ncb = min(CB, NB - cb0);              // packed column blocks of this unit
   bool ok = true;
 
   if (warp == PF_COPY_WARP) {
-    // ---------------- packed weights: HBM -> the packed ring, as far ahead as the ring allows ----------------
-    if (lane == 0) {
-      const uint8_t* wsrc = W + ((size_t)e * NB + cb0) * KG * (size_t)(M * BLOCK_BYTES);
-      const size_t cb_stride = (size_t)KG * (M * BLOCK_BYTES);
-      for (int g = 0; g < KG && ok; ++g) {
-        const int s = g % SP, round = g / SP;
-        if (round > 0) ok = mbar_wait(packed_free + s, (round - 1) & 1);
-        if (!ok) break;
-        uint8_t* dst = smem + SM::PACKED_OFFSET + s * SM::PACKED_BYTES;
-        mbar_expect_tx(packed_full + s, (uint32_t)ncb * (M * BLOCK_BYTES));
-        for (int j = 0; j < ncb; ++j)
-          bulk_g2s(dst + j * (M * BLOCK_BYTES), wsrc + j * cb_stride + (size_t)g * (M * BLOCK_BYTES), M * BLOCK_BYTES,
-                   packed_full + s);
-      }
+    // ---------------- packed weights: HBM -> the packed ring, a lane a column block, as far ahead as the ring allows
+    const size_t cb_stride = (size_t)KG * (M * BLOCK_BYTES);
+    const uint8_t* wsrc = W + (size_t)e * NB * cb_stride + (size_t)(cb0 + lane) * cb_stride;
+    int g = 0;
+    for (; g < KG; ++g, wsrc += M * BLOCK_BYTES) {
+      const int s = g % SP, round = g / SP;
+      if (round > 0) ok = mbar_wait_warp(packed_free + s, (round - 1) & 1);
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(packed_full + s, (uint32_t)ncb * (M * BLOCK_BYTES));
+      __syncwarp();
+      if (lane < ncb)
+        bulk_g2s(smem + SM::PACKED_OFFSET + s * SM::PACKED_BYTES + lane * (M * BLOCK_BYTES), wsrc, M * BLOCK_BYTES,
+                 packed_full + s);
     }
+    if (!ok && lane == 0)                            // give the copies in flight a while to land
+      for (int f = max(0, g - SP); f < g; ++f) mbar_wait_for(packed_full + f % SP, (f / SP) & 1, 10000000ull);
     __syncwarp();
   } else if (warp == PF_MMA_WARP) {
     // ---------------- MMA issue: one lane ----------------
     if (lane == 0) {
       const uint32_t idesc = umma_idesc(nmma);
+      const uint64_t desc0 = umma_desc(smem_addr(smem));       // addresses count 16 bytes
+      int s = 0, ph = 0;
       for (int g = 0; g < KG && ok; ++g) {
-        const int s = g % SA, ph = (g / SA) & 1;
-        ok = mbar_wait(a_ready + s, ph) && mbar_wait(b_ready + s, ph);
+        ok = mbar_wait(b_ready + s, ph) && mbar_wait(a_ready + (g & 1), (g >> 1) & 1);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t abase = smem_addr(smem + s * SM::AB_BYTES), bbase = abase + M * SM::A_BYTES;
+        const uint64_t desc = desc0 + (uint32_t)(s * (b_bytes >> 4));
+        const uint32_t a = tmem_base + PF_A_COL + (g & 1) * 32;
 #pragma unroll
-        for (int m = 0; m < M; ++m)
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma(tmem_base + m * 256, umma_desc(abase + m * SM::A_BYTES + ks * 32), umma_desc(bbase + ks * 32), idesc,
-                 (g | ks) ? 1u : 0u);
-        umma_commit(ab_free + s);
+        for (int ks = 0; ks < 4; ++ks) umma_ta(tmem_base, a + ks * 8, desc + 2 * ks, idesc, (g | ks) ? 1u : 0u);
+        umma_commit(a_free + (g & 1));
+        umma_commit(b_free + s);
+        if (++s == sb) {
+          s = 0;
+          ph ^= 1;
+        }
       }
       if (ok) umma_commit(acc_ready);
     }
@@ -230,96 +264,137 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
       rowp[j] = p < 0 ? nullptr : X + (size_t)(slots ? p / slots : p) * x_stride + c * 8;
     }
     const uint32_t boff = (uint32_t)(r0 * 128 + ((c ^ (r0 & 7)) << 4));      // rows 16 apart share r & 7
+    int s = 0, ph = 1, back = 0;                     // ph: a ring's first round finds every stage free
     for (int g = 0; g < KG && ok; ++g) {
-      const int s = g % SA, round = g / SA;
-      if (round > 0) ok = mbar_wait_warp(ab_free + s, (round - 1) & 1);
+      if (g >= sb) ok = mbar_wait_warp(b_free + s, ph);
       if (!ok) break;
-      uint8_t* btile = smem + s * SM::AB_BYTES + M * SM::A_BYTES + boff;
+      uint8_t* btile = smem + s * b_bytes + boff;
 #pragma unroll
-      for (int j = 0; j < PF_GA_PER_THREAD; ++j)
+      for (int j = 0; j < PF_GA_PER_THREAD; ++j) {
+        if (16 * j >= cnt) break;
         if (rowp[j]) cp_async16(btile + j * (16 * 128), rowp[j] + g * GS);
+      }
       cp_async_commit();
-      if (g > 0) {                                   // the stage before this one has landed: publish it
+      if (++s == sb) {
+        s = 0;
+        ph ^= 1;
+      }
+      if (g >= 1) {                                  // the stage before this one has landed: publish it
         cp_async_wait<1>();
         fence_async_smem();
-        mbar_arrive(b_ready + (g - 1) % SA);
+        mbar_arrive(b_ready + back);
+        if (++back == sb) back = 0;
       }
     }
     cp_async_wait<0>();
     fence_async_smem();
-    if (ok) mbar_arrive(b_ready + (KG - 1) % SA);
+    if (ok) mbar_arrive(b_ready + back);
   } else {
-    // ---------------- warps 0-7: dequantise into the A tiles ----------------
-    // warp -> packed column block cbw = warp & 3 and its 16-column tile tt = warp >> 2, for every matrix
-    const int gq = lane >> 2, t = lane & 3, cbw = warp & 3, tt = warp >> 2;
-    for (int g = 0; g < KG && ok; ++g) {
-      const int sp = g % SP, sa = g % SA;
+    // ---------------- warps 0-7: dequantise into the A stages ----------------
+    // A lane holds one weight row: tensor-memory lanes 32 q .. 32 q + 31 belong to warps q and q + 4.  Lane 4 gq + t
+    // takes column 8 (t & 1) + gq of a 16-column tile; t >> 1 picks the tile (one matrix: of the two of column block
+    // q) or the matrix (gate / up: of tile q & 1 of column block q >> 1).
+    // A row's 64 nibbles are four 8-byte pieces, 16 bytes apart; the lanes read them in rotated orders so that a half
+    // warp's loads touch every bank once (in the same order they were a four-way conflict), and the rotation is
+    // undone in registers.
+    const int gq = lane >> 2, t = lane & 3, q = warp & 3, set = warp >> 2;
+    const int cbw = M == 1 ? q : q >> 1, tt = M == 1 ? t >> 1 : q & 1, mm = M == 1 ? 0 : t >> 1, hi = t & 1;
+    const int rot = (t >> 1) * 2 + ((gq >> 1) & 1);
+    const int at = cbw * (M * BLOCK_BYTES) + mm * BLOCK_BYTES;
+    const int w_at = at + tt * TILE_BYTES + gq * 64 + hi * 8, sb_at = at + SB_OFFSET + gq * 16 + (2 * tt + hi) * 4;
+    const uint32_t a_dst = tmem_base + ((uint32_t)(q * 32) << 16) + PF_A_COL + set * 32;
+    for (int g = set; g < KG && ok; g += 2) {
+      const int sp = g % SP;
       ok = mbar_wait_warp(packed_full + sp, (g / SP) & 1);
-      if (ok && g >= SA) ok = mbar_wait_warp(ab_free + sa, (g / SA - 1) & 1);
       if (!ok) break;
+      const uint8_t* blk = smem + SM::PACKED_OFFSET + sp * SM::PACKED_BYTES;
+      uint2 w[4];
+      uint32_t sbw = 0u;
       if (cbw < ncb) {
-        const uint8_t* blk = smem + SM::PACKED_OFFSET + sp * SM::PACKED_BYTES + cbw * (M * BLOCK_BYTES);
+        sbw = *reinterpret_cast<const uint32_t*>(blk + sb_at);
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-          const uint4 sbv = *reinterpret_cast<const uint4*>(blk + m * BLOCK_BYTES + SB_OFFSET + gq * 16);
-          const uint4 w = *reinterpret_cast<const uint4*>(blk + m * BLOCK_BYTES + tt * TILE_BYTES + lane * 16);
-          const uint32_t sb_lo = comp(sbv, 2 * tt), sb_hi = comp(sbv, 2 * tt + 1);
-          // rows of the A tile: column cbw * 32 + tt * 16 + gq (and + 8); chunks 2 t and 2 t + 1 of the row
-          uint8_t* row = smem + sa * SM::AB_BYTES + m * SM::A_BYTES + (cbw * 32 + tt * 16 + gq) * 128;
+        for (int u = 0; u < 4; ++u) w[u] = *reinterpret_cast<const uint2*>(blk + w_at + (((u + rot) & 3) << 4));
+      } else {
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const uint32_t word = comp(w, h);
-            const uint32_t sb = (h & 2) ? sb_hi : sb_lo;
-            uint4 o;
-            o.x = prefill_pair<SB>(nib_pair(word, 0), sb);
-            o.y = prefill_pair<SB>(nib_pair(word, 4), sb);
-            o.z = prefill_pair<SB>(nib_pair(word, 8), sb);
-            o.w = prefill_pair<SB>(nib_pair(word, 12), sb);
-            const int chunk = 2 * t + (h & 1);
-            *reinterpret_cast<uint4*>(row + (h & 2) * 512 + ((chunk ^ gq) << 4)) = o;
-          }
-        }
+        for (int u = 0; u < 4; ++u) w[u] = make_uint2(0u, 0u);
       }
-      fence_async_smem();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(packed_free + sp);
-        mbar_arrive(a_ready + sa);
+      if (lane == 0) mbar_arrive(packed_free + sp);
+      uint2 v[4], x[4];                              // piece k = w[(k - rot) & 3]
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = (rot & 1) ? w[(k + 3) & 3] : w[k];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = (rot & 2) ? v[(k + 2) & 3] : v[k];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {                  // half a row: 32 inputs, 16 columns
+        uint32_t o[16];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t word = i & 1 ? x[2 * h + (i >> 1)].y : x[2 * h + (i >> 1)].x;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[4 * i + j] = prefill_pair<SB>(nib_pair(word, 4 * j), sbw);
+        }
+        if (h == 0 && g >= 2) {
+          ok = mbar_wait_warp(a_free + set, ((g >> 1) - 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        tmem_st16(a_dst + 16 * h, o);
       }
+      if (!ok) break;
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(a_ready + set);
     }
   }
   // ---------------- epilogue: the twelve dequantising and gathering warps ----------------
-  // TMEM lane quarter warp & 3 (output column (warp & 3) * 32 + lane of the unit); the three warps of a quarter take
-  // a third of the pairs each, 16 pairs a load
+  // TMEM lane quarter warp & 3, a weight row a lane (numbered as the dequantising warps do); the three warps of a
+  // quarter take a third of the pairs each, 16 pairs a load.  Gate and up rows of a column sit in lanes 2 apart: of
+  // two neighbouring pairs the gate lane forms the first and the up lane the second, one exchange for both.
   if (warp < PF_DQ_WARPS + PF_GA_WARPS) {
     if (ok) ok = mbar_wait_warp(acc_ready, 0);
     if (ok) {
       tc_fence_after();
-      const int q = warp & 3, part = warp >> 2, col = ct * PF_COLS + q * 32 + lane;
+      const int q = warp & 3, part = warp >> 2, gq = lane >> 2, t = lane & 3;
+      const int col = M == 1 ? ct * PF_ROWS + q * 32 + (t >> 1) * 16 + (t & 1) * 8 + gq
+                             : ct * (PF_ROWS / 2) + q * 16 + (t & 1) * 8 + gq;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
       const int blocks = nmma / 16, per = (blocks + 2) / 3;
       const int jb = min(blocks, part * per) * 16, je = min(blocks, (part + 1) * per) * 16;
       for (int j0 = jb; j0 < je; j0 += 16) {
-        uint32_t a[16], b[16];
+        uint32_t a[16];
         tmem_ld16(taddr + j0, a);
-        if constexpr (M == 2) tmem_ld16(taddr + 256 + j0, b);
         tmem_ld_wait();
-        if (col < N) {
-          // the sixteen values first (independent chains the compiler can interleave: one after the other, each
-          // behind its own row lookup and branch, they took 2 us a block), then their rows and the stores
+        // the values first (independent chains the compiler can interleave: one after the other, each behind its own
+        // row lookup and branch, they took 2 us a block), then their rows and the stores
+        if constexpr (M == 2) {
+          static_assert(EPI == EPI_SWIGLU, "two matrices: gate and up");
+          const bool up_lane = (t & 2) != 0;
+          float r[8];
+          int rows[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float give = __uint_as_float(up_lane ? a[2 * j] : a[2 * j + 1]);
+            const float keep = __uint_as_float(up_lane ? a[2 * j + 1] : a[2 * j]);
+            const float got = __shfl_xor_sync(0xffffffffu, give, 2);
+            rows[j] = out_row[j0 + 2 * j + (up_lane ? 1 : 0)];
+            r[j] = swiglu_fast(up_lane ? got : keep, up_lane ? keep : got, limit);
+          }
+          if (col < N) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (rows[j] >= 0)
+                static_cast<__nv_bfloat16*>(out)[(size_t)rows[j] * N + col] = __float2bfloat16_rn(r[j]);
+          }
+        } else if (col < N) {
           float r[16];
           int rows[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const float v = __uint_as_float(a[j]);
             rows[j] = out_row[j0 + j];
-            if constexpr (EPI == EPI_RELU2) {
-              r[j] = relu2(v);
-            } else if constexpr (EPI == EPI_SWIGLU) {
-              r[j] = swiglu_fast(v, __uint_as_float(b[j]), limit);
-            } else {
-              r[j] = v;
-            }
+            r[j] = EPI == EPI_RELU2 ? relu2(v) : v;
           }
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
@@ -338,14 +413,14 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
   pdl_launch_dependents();
   tc_fence_before();
   __syncthreads();
-  if (warp == PF_MMA_WARP) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (warp == PF_MMA_WARP) tmem_dealloc(tmem_base, PF_TMEM_COLS);
 }
 
 template <int M, int EPI, int SB>
 int launch_prefill(const void* x, int64_t x_stride, int slots, const void* w, int kg, int nb, const int* items,
                    const int* counts, const int* members, void* out, int n, float limit, int64_t max_items,
                    cudaStream_t stream) {
-  using SM = PrefillSmem<M>;
+  using SM = PrefillSmem;
   auto* kern = prefill_kernel<M, EPI, SB>;
   static bool configured[64] = {false};
   int dev = 0;
@@ -356,7 +431,7 @@ int launch_prefill(const void* x, int64_t x_stride, int slots, const void* w, in
              "experts_prefill: shared memory opt-in");
     configured[dev] = true;
   }
-  const int64_t grid = max_items * ((nb + PF_CB - 1) / PF_CB);
+  const int64_t grid = max_items * ((nb + PF_CB<M> - 1) / PF_CB<M>);
   if (grid >= (int64_t(1) << 31)) return fail(TFB_ERR_ARG, "experts_prefill: too many units");
   return check_cuda(launch(kern, dim3((unsigned)grid), dim3(PF_THREADS), (size_t)SM::TOTAL, stream,
                            static_cast<const __nv_bfloat16*>(x), x_stride, slots, static_cast<const uint8_t*>(w), kg,

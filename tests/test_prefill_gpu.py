@@ -126,3 +126,40 @@ def test_prefill_layer_against_the_oracle(shared, pdl):
     assert rel_l2(out.float().cpu().numpy(), o64) <= 1e-2
     dec = moe.run(x, layer)                                        # the decode form agrees within the same tolerance
     assert rel_l2(out.float().cpu().numpy(), dec.float().cpu().numpy()) <= 1e-2
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 191, 192, 193])
+@pytest.mark.parametrize("width, dims", [(32, 64), (96, 128), (160, 192)])
+def test_tile_edges_equal_the_rounded_weights_product(rows, width, dims, dtype):
+    """Items around the MMA's row granularity and capacity, column counts that leave a unit's blocks missing (one matrix:
+    128 columns a unit, gate and up: 64) and one to three groups of inputs, one expert.  Bounds: the gate/up output is
+    within two bf16 roundings (2^-7) of the rounded reference's largest value, the fp32 down product within the error of a
+    K <= 192 fp32 sum (1e-5 of the largest value)."""
+
+    from tensorfold_b200 import _lib, experts
+
+    gate, up = mlx(1, width, dims, 5, dtype), mlx(1, width, dims, 6, dtype)
+    ex = experts.make([gate, up], mlx(1, dims, 64, 7, dtype), 64)  # (the down projection is not run)
+    x = (torch.randn((rows, dims), generator=torch.Generator().manual_seed(rows)) * 0.5).to(torch.bfloat16).to(DEV)
+    plan = experts.Plan(rows, 1, 1, DEV, prefill=True)
+    experts.route(torch.zeros((rows, 1), dtype=torch.int32, device=DEV), plan)
+    act = torch.full((rows, width), float("nan"), dtype=torch.bfloat16, device=DEV)
+    experts.gate_up(x, ex, plan, act, rows)
+    torch.cuda.synchronize()
+    assert _lib.kernel_status() == 0
+
+    def weights(m):
+        return dequant64(*m)[0].float().to(torch.bfloat16).double()
+
+    g, u = (x.double() @ weights(m).T for m in (gate, up))
+    g, u = g.float().to(torch.bfloat16).double(), u.float().to(torch.bfloat16).double()
+    ref = (g * torch.sigmoid(g)).to(torch.bfloat16).double() * u
+    assert (act.double() - ref).abs().max() <= 2 ** -7 * ref.abs().max()
+    y = torch.full((rows, width), float("nan"), dtype=torch.float32, device=DEV)
+    single = experts.pack(*gate, 64).unsqueeze(3)                  # one matrix: fp32 rows of the gate projection
+    experts._run(0, x, 1, single, dims // 64, width // 32, plan, y, width, 0.0,
+                 experts.max_items(rows, 1, plan.tile), ex, True)
+    torch.cuda.synchronize()
+    ref = x.double() @ weights(gate).T
+    assert _lib.kernel_status() == 0 and (y.double() - ref).abs().max() <= 1e-5 * ref.abs().max()
