@@ -97,24 +97,34 @@ __device__ __forceinline__ void lane_words(const uint32_t* __restrict__ tile, in
   }
 }
 
-// st[j] = state of value 8 lane + j from the lane's words.
-template <int K2>
+// A 16-bit half of a word, zero-extended.  MUL: by a two-way dot product (times 1 and 0), which runs on the multiply
+// pipe; else by a byte permute on the ALU pipe.  Both pipes take one instruction every two cycles a scheduler and the
+// decode is bound by the fuller one, so the states' extraction is split between them: 4.00 bits 23 ALU + 16 multiply ->
+// 19 + 20 (61 -> 54 cycles a tile in a loop of its own), the other widths 28-30 + 16 -> 22 + 24 (71 -> 64).
+template <bool MUL>
+__device__ __forceinline__ uint32_t half_hi(uint32_t w) {
+  return MUL ? __dp2a_lo(w, 0x0100u, 0u) : prmt(w, 0u, 0x4432);
+}
+template <bool MUL>
+__device__ __forceinline__ uint32_t half_lo(uint32_t w) {
+  return MUL ? __dp2a_lo(w, 0x0001u, 0u) : prmt(w, 0u, 0x4410);
+}
+
+// st[j] = state of value 8 lane + j from the lane's words.  MUL: the multiply pipe has room (not with a codebook that
+// uses it for a byte sum).
+template <int K2, bool MUL>
 __device__ __forceinline__ void lane_states(const uint32_t (&w)[Win<K2>::NW], int lane, uint32_t (&st)[8]) {
   constexpr int NW = Win<K2>::NW, NV = Win<K2>::NV;
   if constexpr (K2 == 8) {
-    // 16-bit windows ending 4 (j + 1) bits into the lane's own word w[1], the stream running on from w[0].  Three
-    // funnel shifts line the windows up on byte boundaries; a byte permute then cuts each one out, zero-extended.
-    const uint32_t q16 = __funnelshift_r(w[1], w[0], 16);           // stream bits -16 .. 16 of the own word
-    const uint32_t q20 = __funnelshift_r(w[1], w[0], 20);           // -20 .. 12
-    const uint32_t q4 = __funnelshift_r(w[1], w[0], 4);             // -4 .. 28
-    st[0] = prmt(q20, 0u, 0x4421);                                  // bits -12 .. 4
-    st[1] = prmt(q16, 0u, 0x4421);                                  // -8 .. 8
-    st[2] = prmt(q20, 0u, 0x4410);                                  // -4 .. 12
-    st[3] = prmt(q16, 0u, 0x4410);                                  // 0 .. 16
-    st[4] = prmt(q4, 0u, 0x4421);                                   // 4 .. 20
-    st[5] = prmt(w[1], 0u, 0x4421);                                 // 8 .. 24
-    st[6] = prmt(q4, 0u, 0x4410);                                   // 12 .. 28
-    st[7] = prmt(w[1], 0u, 0x4410);                                 // 16 .. 32
+    // 16-bit windows ending 4 (j + 1) bits into the lane's own word w[1], the stream running on from w[0]: a word that
+    // starts with window j ends with window j + 4
+    const uint32_t t[4] = {__funnelshift_l(w[1], w[0], 20), __funnelshift_l(w[1], w[0], 24),
+                           __funnelshift_l(w[1], w[0], 28), w[1]};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      st[j] = half_hi<false>(t[j]);
+      st[j + 4] = half_lo<MUL>(t[j]);
+    }
   } else {
     const int off = (4 * lane * K2 + (K2 >> 1) - 16 + 32 * Win<K2>::TW) & 31;
     uint32_t v[NV];                                   // v[i] = stream bits [first + 32 i, first + 32 i + 32)
@@ -123,10 +133,17 @@ __device__ __forceinline__ void lane_states(const uint32_t (&w)[Win<K2>::NW], in
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int d = delta<K2>(j), i = d >> 5, o = d & 31;
-      if (o <= 16) {
-        st[j] = (v[i] >> (16 - o)) & 0xFFFFu;
-      } else {                                        // the window runs into the next chunk (d + 16 <= SPAN: it exists)
-        st[j] = __funnelshift_l(v[i + 1 < NV ? i + 1 : i], v[i], o) >> 16;
+      const uint32_t next = v[i + 1 < NV ? i + 1 : i];   // o > 16: the window runs into it (d + 16 <= SPAN: it exists)
+      if (o == 0) {
+        st[j] = half_hi<MUL>(v[i]);
+      } else if (o == 16) {
+        st[j] = half_lo<MUL>(v[i]);
+      } else if (o == 8) {                            // on a byte boundary: one permute cuts it out
+        st[j] = prmt(v[i], 0u, 0x4421);
+      } else if (o < 16) {
+        st[j] = half_lo<MUL>(v[i] >> (16 - o));
+      } else {
+        st[j] = half_hi<MUL>(__funnelshift_l(next, v[i], o));
       }
     }
   }
@@ -138,7 +155,7 @@ __device__ __forceinline__ void lane_states(const uint32_t (&w)[Win<K2>::NW], in
 template <int CB, int K2>
 __device__ __forceinline__ void decode_words(const uint32_t (&w)[Win<K2>::NW], int lane, uint32_t (&a)[4]) {
   uint32_t st[8];
-  lane_states<K2>(w, lane, st);
+  lane_states<K2, CB != 2>(w, lane, st);
   a[0] = cb_pair<CB>(st[0], st[1]);
   a[2] = cb_pair<CB>(st[2], st[3]);
   a[1] = cb_pair<CB>(st[4], st[5]);
