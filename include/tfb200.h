@@ -283,8 +283,8 @@ int tfb_exl3_prologue(const void* x, int64_t x_stride, int x_is_fp16, const int3
  * items / counts / members: the prologue's sort; z: fp32 scratch [2, P, N]; arrive: int32 scratch
  * [max_items * N / 128], zero before the first call (a call leaves it zero); max_items >= the sort's item count.
  * sorted_g / sorted_u (both or neither): the prologue's width-ordered items of the two matrices, [., 4] each.
- * item_pairs: 16 or 32, the most pairs an item holds (with 32 one decode of a weight tile serves up to 32 pairs, at
- * more registers a thread: for calls with many pairs an expert); a pair's bits do not depend on it.
+ * item_pairs: 16 or 32, the most pairs an item holds (with 32 one decode of a weight tile serves up to 32 pairs,
+ * in the tensor-memory form of the kernel: for calls with many pairs an expert); a pair's bits do not depend on it.
  * k2_all: 0, or the width every entry of k2_g and k2_u has - a promise that lets the launch use a kernel built for
  * that width alone (a tenth of the code; it pays at a few tokens); a tensor of another width then sets the status
  * word and nothing is stored.  -1: the widths differ - the launch uses a build with short loops, so that blocks

@@ -8,13 +8,15 @@
 // The layer is y = (((x * suh) H) W_q) H * svh per 128-block, H = 128-point Hadamard / sqrt(128).
 //
 // Three launches a layer call (src/tensorfold/cuda/exl3/experts.py:173-202 needs seven):
-//   prologue  one block sorts the (row, slot) pairs by expert into items of <= 16 pairs (the affine plan's sort), the
-//             others rotate every routed pair's input for gate and up (x * suh, 128-point transform, fp16);
+//   prologue  one block sorts the (row, slot) pairs by expert into items of <= 16 or 32 pairs (the affine plan's sort),
+//             the others rotate every routed pair's input for gate and up (x * suh, 128-point transform, fp16);
 //   gate/up   CTA = (item, 64 columns, matrix): the four warps split K, each pulls its rows of tiles through a private
 //             shared-memory ring with bulk async copies, decodes from shared memory and multiplies; the K slices meet
 //             in warp order; the LAST of the four CTAs that share (item, 128 columns) - counted with an atomic - runs
 //             the epilogue (rotate, svh, SwiGLU, suh_d, rotate) for the block and stores the down projection's input;
 //   down      the same kernel with the output rotation (and svh) as its epilogue; y fp32 per pair.
+// Calls with many pairs an expert sort into items of <= 32 pairs, which a second form of the kernel takes
+// (grouped_tc_kernel: 128 columns a CTA, decoded tiles go to tensor memory, tcgen05.mma multiplies): the same sums.
 // Fixed-order reductions everywhere: a pair's bits never depend on the other rows of the call.
 // (Replaces src/tensorfold/cuda/exl3/experts.cu and experts_grouped.cuh; the trellises are read in place.)
 
@@ -30,11 +32,22 @@ constexpr float HAD_SCALE = 0.08838834764831845f;   // 1 / sqrt(128)
 constexpr int GR_WARPS = 4;                         // K slices a CTA (part of the arithmetic: they meet in warp order)
 constexpr int GR_NTB = 4;                           // 16-column tiles a CTA: 64 columns (2: the narrow CTAs, 32 columns)
 constexpr int GR_NARROW_NTB = 2;
-constexpr int GR_PT = 2;                            // mma tiles of 8 pairs an item: 16 pairs (4: the wide items, 32 pairs)
+constexpr int GR_PT = 2;                            // mma tiles of 8 pairs an item: 16 pairs
 constexpr int GR_PAIRS = 8 * GR_PT;
-constexpr int GR_WIDE_PT = 4;
 constexpr int GR_SLOT_BYTES = 2048;                 // a ring slot: whole rows of the CTA's four tiles
 constexpr int GR_STAGES = 3;
+
+// the tensor-memory kernel (the wide items)
+constexpr int TC_SETS = 4;                          // sets of four decoding warps; a set takes every fourth step
+constexpr int TC_DEC_WARPS = 4 * TC_SETS;           // warps 0-15: decode, then the epilogue
+constexpr int TC_LOAD_WARP = TC_DEC_WARPS, TC_MMA_WARP = TC_DEC_WARPS + 1;
+constexpr int TC_THREADS = (TC_DEC_WARPS + 2) * 32;
+constexpr int TC_COLS = 128;                        // output columns a CTA (MMA M), one rotation block
+constexpr int TC_PAIRS = 32;                        // the most pairs an item holds (MMA N)
+constexpr int TC_STEP = 64;                         // inputs a step; a stage of the rings: two steps
+constexpr int TC_PARTS = 4;                         // parts of K, an accumulator each (part of the arithmetic)
+constexpr int TC_A_COL = TC_PARTS * TC_PAIRS;  // tensor memory: the accumulators, then an A stage a set
+constexpr int TC_TMEM_COLS = TC_A_COL + 32 * TC_SETS;
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) { return __byte_perm(a, b, sel); }
 
@@ -268,6 +281,94 @@ __device__ __forceinline__ bool warp_rows(const uint8_t* __restrict__ T, int nti
   return true;
 }
 
+// Two k-tiles of a 16-column tile go to tensor memory as the MMA's A operand: 16 lanes (columns) x 128
+// bits a repeat, register 2 r = (lane g, 32-bit column 4 r + t), 2 r + 1 = (lane g + 8, the same) - which is where a
+// decoded tile's four registers already are.
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_t (&a)[2][4]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(taddr),
+               "r"(a[0][0]), "r"(a[0][1]), "r"(a[0][2]), "r"(a[0][3]), "r"(a[1][0]), "r"(a[1][1]), "r"(a[1][2]),
+               "r"(a[1][3])
+               : "memory");
+}
+
+// Shared memory of a CTA: the trellis ring (stages of 128 inputs x 128 columns: 1024 K2 bytes), the B ring (32 pairs x
+// 128 inputs a stage, two 128-byte-swizzled tiles), the pair table, barriers.  After the main loop the trellis ring's
+// memory takes the accumulators ([32][128] fp32) and, in a cluster, the other parts'.
+struct TrellisSmem {
+  static constexpr int RING_BYTES = 65536, SP_MAX = 8;
+  static constexpr int B_TILE = TC_PAIRS * 128, SB = 4;
+  static constexpr int B_OFFSET = RING_BYTES;
+  static constexpr int PAIR_OFFSET = B_OFFSET + SB * 2 * B_TILE;
+  static constexpr int BAR_OFFSET = PAIR_OFFSET + TC_PAIRS * 4;
+  static constexpr int NBARS = 2 * SP_MAX + 2 * TC_SETS + 2 * SB + 1;
+  static constexpr int FLAG_OFFSET = BAR_OFFSET + NBARS * 8;     // tensor-memory address, last-arrival flag
+  static constexpr int TOTAL = FLAG_OFFSET + 16 + 1024;          // + slack to align the tiles to 1024 bytes
+};
+static_assert(TC_PARTS * TC_PAIRS * TC_COLS * 4 <= TrellisSmem::RING_BYTES, "every part's accumulators fit the ring");
+static_assert(2 * (TrellisSmem::TOTAL + 1024) <= 228 * 1024 && 2 * TC_TMEM_COLS <= 512, "two CTAs share an SM");
+
+template <int K2>
+struct Ring {
+  static constexpr int STAGE_BYTES = 2 * TC_STEP / 16 * (TC_COLS / 16) * 16 * K2;
+  static constexpr int SP = K2 <= 8 ? 8 : 4;
+  static_assert(SP * STAGE_BYTES <= TrellisSmem::RING_BYTES && SP <= TrellisSmem::SP_MAX, "the ring holds its stages");
+};
+
+// One decoding warp's share of the CTA's steps of 64 inputs: warp q of a set takes the column tiles 2 q and 2 q + 1
+// (tensor-memory lanes 32 q ..) of the set's steps.  Returns false when a wait ran out.
+template <int CB, int K2>
+__device__ __forceinline__ bool decode_stages(const uint8_t* ring, uint64_t* packed_full, uint64_t* packed_free,
+                                              uint64_t* a_ready, uint64_t* a_free, uint32_t a_dst, int set, int q,
+                                              int steps, int lane) {
+  constexpr int TW = Win<K2>::TW, NW = Win<K2>::NW, SP = Ring<K2>::SP;
+  // where the lane's words sit inside a tile: NW consecutive words (cyclically) from the one that holds the first bit
+  // of value 8 lane's window
+  int word[NW];
+  {
+    int wi = ((4 * lane * K2 + (K2 >> 1) - 16 + 32 * TW) >> 5) % TW;
+#pragma unroll
+    for (int j = 0; j < NW; ++j) {
+      word[j] = wi + ((set & 1) * (TC_STEP / 16) * (TC_COLS / 16) + 2 * q) * TW;   // odd sets: a stage's second step
+      wi = wi + 1 == TW ? 0 : wi + 1;
+    }
+  }
+  for (int g = set, use = 0; g < steps; g += TC_SETS, ++use) {
+    const int p = g >> 1, sp = p % SP;
+    if (!mbar_wait_warp(packed_full + sp, (p / SP) & 1)) return false;
+    if (use > 0) {
+      if (!mbar_wait_warp(a_free + set, (use - 1) & 1)) return false;
+      tc_fence_after();
+    }
+    const uint32_t* stage = reinterpret_cast<const uint32_t*>(ring + sp * Ring<K2>::STAGE_BYTES);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t a[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t* tile = stage + ((2 * h + i) * (TC_COLS / 16) + c) * TW;
+          uint32_t w[NW];
+#pragma unroll
+          for (int j = 0; j < NW; ++j) w[j] = tile[word[j]];
+          uint32_t v[4];
+          decode_words<CB, K2>(w, lane, v);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) a[i][j] = v[j];
+        }
+        tmem_st_16x128b_x4(a_dst + ((uint32_t)(16 * c) << 16) + 16 * h, a);
+      }
+    }
+    __syncwarp();
+    mbar_arrive_if(packed_free + sp, lane == 0);
+    tmem_st_wait();
+    tc_fence_before();
+    __syncwarp();
+    mbar_arrive_if(a_ready + set, lane == 0);
+  }
+  return true;
+}
+
 // ---- 128-point Walsh-Hadamard transform by 16 lanes, 8 consecutive values a lane ---------------------------------
 // Strides 1, 2, 4 inside the lane, 8 .. 64 across the 16 lanes of a half warp (sub = lane % 16); a warp transforms two
 // blocks at once.  Not scaled.
@@ -309,6 +410,10 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {   // anot
   const float4 a = __ldcg(reinterpret_cast<const float4*>(p)), b = __ldcg(reinterpret_cast<const float4*>(p) + 1);
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
+__device__ __forceinline__ void load8_shared(const float* p, float (&f)[8]) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
 __device__ __forceinline__ void store8(__half* p, const float (&f)[8], float scale) {
   uint4 u;
   __half2* h = reinterpret_cast<__half2*>(&u);
@@ -320,12 +425,10 @@ __device__ __forceinline__ void store8(__half* p, const float (&f)[8], float sca
 // ---- epilogues of one pair and one 128-block, by a half warp ------------------------------------------------------
 // gate/up: rotate both, * svh, SwiGLU (act_mode 0: the GLM family's bf16 roundings; 1: fp32), * suh_d, rotate, fp16.
 // (arithmetic of src/tensorfold/cuda/exl3/experts.cu:116-158)
-__device__ __forceinline__ void gateup_block(const float* zg, const float* zu, const __half* svh_g, const __half* svh_u,
+__device__ __forceinline__ void gateup_block(float (&g)[8], float (&u)[8], const __half* svh_g, const __half* svh_u,
                                              const __half* suh_d, __half* xd, int sub, float limit, int act_mode,
                                              bool store) {
-  float g[8], u[8], sg[8], su[8], sd[8];
-  load8(zg + 8 * sub, g);
-  load8(zu + 8 * sub, u);
+  float sg[8], su[8], sd[8];
   load8(svh_g + 8 * sub, sg);
   load8(svh_u + 8 * sub, su);
   load8(suh_d + 8 * sub, sd);
@@ -350,9 +453,8 @@ __device__ __forceinline__ void gateup_block(const float* zg, const float* zu, c
 }
 
 // down: y = rotate(z) * svh, fp32.  (src/tensorfold/cuda/exl3/experts.cu:161-180)
-__device__ __forceinline__ void down_block(const float* z, const __half* svh, float* y, int sub, bool store) {
-  float v[8], s[8];
-  load8(z + 8 * sub, v);
+__device__ __forceinline__ void down_block(float (&v)[8], const __half* svh, float* y, int sub, bool store) {
+  float s[8];
   load8(svh + 8 * sub, s);
   hadamard128(v, sub);
   if (!store) return;
@@ -375,7 +477,7 @@ struct GroupedArgs {
   const __half* x[2];            // rotated inputs [P, K] fp16 of matrix 0 / 1
   const int64_t* tp[2];          // trellis pointers [E]
   const int* k2[2];              // half-bit widths [E]
-  const int* items;              // [., 3] (expert, first, count <= 16)
+  const int* items;              // [., 3] (expert, first, count <= 32)
   const int* sorted[2];          // or null: the items in the order their CTAs should run, [., 4] = (expert, first, count, index)
   const int* counts;             // [0] = items
   const int* members;            // pair ids p = row * slots + slot, grouped by expert
@@ -385,21 +487,21 @@ struct GroupedArgs {
   const __half* suh_next;        // gate/up: suh of the down projection [E, N]
   void* out;                     // gate/up: xd [P, N] fp16; down: y [P, N] fp32
   int K, N, P, mats, epi, act_mode;
+  int k2_all;                    // 8: every tensor has 4.00 bits (a promise); else 0
   float limit;
 };
 
 enum GroupedEpilogue : int { GE_NONE = 0, GE_GATEUP = 1, GE_DOWN = 2 };
 
-// CTA (item, 64 columns, matrix).  PT: mma tiles of eight pairs an item may hold (2: items of 16 pairs; 4: items of 32,
-// for calls with many pairs an expert - every weight tile is then decoded once for up to 32 pairs).
+// CTA (item, 64 columns, matrix), items of up to 16 pairs.
 // K2F: 0, or the one width every tensor of the launch has (the host knows it): the kernel then holds that width's loop
 // alone - a tenth of the code, which matters where a CTA's life is short (one token: the dominant stall of the
 // all-widths kernel was the instruction fetch).
 // NTB: 16-column tiles a CTA (4, or 2 where the launch would otherwise have too few CTAs to fill the GPU).
-template <int CB, int PT, int K2F, int NTB, bool COMPACT>
+template <int CB, int K2F, int NTB, bool COMPACT>
 __global__ void __launch_bounds__(GR_WARPS * 32)
 grouped_kernel(const GroupedArgs a) {
-  constexpr int PAIRS = 8 * PT, GR_RED_STRIDE = NTB * 16 + 1;
+  constexpr int PT = GR_PT, PAIRS = GR_PAIRS, GR_RED_STRIDE = NTB * 16 + 1;
   constexpr int RING_BYTES = GR_WARPS * GR_STAGES * GR_SLOT_BYTES, RED_BYTES = GR_WARPS * PAIRS * GR_RED_STRIDE * 4;
   // the K slices meet in the ring's memory (free by then)
   __shared__ __align__(128) uint8_t ring[RING_BYTES > RED_BYTES ? RING_BYTES : RED_BYTES];
@@ -450,13 +552,9 @@ grouped_kernel(const GroupedArgs a) {
   bool ok = true;
   uint8_t* my_ring = ring + warp * (GR_STAGES * GR_SLOT_BYTES);
   uint64_t* my_bars = bars + warp * GR_STAGES;
-#define TFB_K2_BODY(K2_)                                                                                  \
-    if constexpr (PT == 2)                                                                                \
-      ok = live > 1 ? warp_rows<CB, K2_, 2, 2, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc)  \
-                    : warp_rows<CB, K2_, 2, 1, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc); \
-    else                                                                                                  \
-      ok = live > 2 ? warp_rows<CB, K2_, 4, 4, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc)  \
-                    : warp_rows<CB, K2_, 4, 2, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc);
+#define TFB_K2_BODY(K2_)                                                                                              \
+    ok = live > 1 ? warp_rows<CB, K2_, PT, PT, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc) \
+                  : warp_rows<CB, K2_, PT, 1, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc);
 #define TFB_K2(K2_) \
   case K2_:         \
     TFB_K2_BODY(K2_) \
@@ -527,11 +625,284 @@ grouped_kernel(const GroupedArgs a) {
     const int p = pair_sh[p0 + half];
     const int q = p < 0 ? pair_sh[0] : p;
     const size_t at = (size_t)q * a.N + blk * 128, sc = (size_t)e * a.N + blk * 128;
-    if (a.epi == GE_GATEUP)
-      gateup_block(a.z + at, a.z + (size_t)a.P * a.N + at, a.sv[0] + sc, a.sv[1] + sc, a.suh_next + sc,
-                   static_cast<__half*>(a.out) + at, sub, a.limit, a.act_mode, p >= 0);
-    else
-      down_block(a.z + at, a.sv[0] + sc, static_cast<float*>(a.out) + at, sub, p >= 0);
+    float g[8], u[8];
+    load8(a.z + at + 8 * sub, g);
+    if (a.epi == GE_GATEUP) {
+      load8(a.z + (size_t)a.P * a.N + at + 8 * sub, u);
+      gateup_block(g, u, a.sv[0] + sc, a.sv[1] + sc, a.suh_next + sc, static_cast<__half*>(a.out) + at, sub, a.limit,
+                   a.act_mode, p >= 0);
+    } else {
+      down_block(g, a.sv[0] + sc, static_cast<float*>(a.out) + at, sub, p >= 0);
+    }
+  }
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+// kind::f16: D fp32, A and B fp16, both K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t umma_idesc_f16(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TC_COLS >> 4) << 24);
+}
+
+// CTA (item, 128 columns, matrix), eighteen warps.  Per stage of 128 inputs: a warp copies the trellis rows into the ring
+// and gathers the pairs' rotated inputs into swizzled B tiles, the decoding warps turn the 64 tiles into fp16 and store
+// them in tensor memory, one lane of the last warp multiplies (A from tensor memory: a tile is decoded once for up to
+// 32 pairs and touches neither shared memory nor further registers).
+// The four parts of K are four accumulators, added in order: the sums of grouped_kernel's four warps, bit for bit.
+//
+// What bounds it: instruction issue in the decode, about 60 instructions a tile and lane with the pipeline's own.
+// Two CTAs of sixteen decoding warps fill an SM's tensor memory.
+// TC_MEASURED
+template <int CB>
+__global__ void __launch_bounds__(TC_THREADS, 2)
+grouped_tc_kernel(const GroupedArgs a) {
+  using SM = TrellisSmem;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  int* pair_sh = reinterpret_cast<int*>(smem + SM::PAIR_OFFSET);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::BAR_OFFSET);
+  uint64_t* packed_full = bars;                       // [SP] the trellis rows of the stage landed
+  uint64_t* packed_free = packed_full + SM::SP_MAX;   // [SP] the decoding warps have read it
+  uint64_t* a_ready = packed_free + SM::SP_MAX;       // [sets] the set's four warps stored their tiles
+  uint64_t* a_free = a_ready + TC_SETS;               // [sets] the MMAs that read the A stage retired
+  uint64_t* b_ready = a_free + TC_SETS;                     // [SB] the pairs' inputs landed
+  uint64_t* b_free = b_ready + SM::SB;                // [SB] the MMAs that read the B stage retired
+  uint64_t* acc_ready = b_free + SM::SB;
+  uint32_t* flags = reinterpret_cast<uint32_t*>(smem + SM::FLAG_OFFSET);   // [0] tensor memory, [1] last
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int blk = blockIdx.x, mat = blockIdx.z;
+  if (tid == 0) {
+    for (int s = 0; s < SM::SP_MAX; ++s) {
+      mbar_init(packed_full + s, 1);
+      mbar_init(packed_free + s, 8);                  // the two sets whose steps the stage holds
+    }
+    for (int s = 0; s < TC_SETS; ++s) {
+      mbar_init(a_ready + s, 4);
+      mbar_init(a_free + s, 1);
+    }
+    for (int s = 0; s < SM::SB; ++s) {
+      mbar_init(b_ready + s, 32);
+      mbar_init(b_free + s, 1);
+    }
+    mbar_init(acc_ready, 1);
+    mbar_fence_init();
+    fence_async_smem();
+  }
+  pdl_wait();
+  const int *items = a.items, *counts = a.counts, *members = a.members, *sorted = a.sorted[mat];
+  const __half* xin = a.x[mat];
+  after_wait(items, counts, members, xin, sorted);
+  // the item is read together with the count that says whether it exists (its slot is always inside the table)
+  const int n_items = ld_dep(counts);
+  int it = blockIdx.y, e, first, cnt;
+  if (sorted != nullptr) {                            // the CTA's place in the launch is not the item's index
+    const int4 s4 = ld_dep4(sorted + 4 * blockIdx.y);
+    e = s4.x, first = s4.y, cnt = min(s4.z, TC_PAIRS), it = s4.w;
+  } else {
+    e = ld_dep(items + 3 * it), first = ld_dep(items + 3 * it + 1), cnt = min(ld_dep(items + 3 * it + 2), TC_PAIRS);
+  }
+  if ((int)blockIdx.y >= n_items) return;
+  const uint8_t* T = reinterpret_cast<const uint8_t*>(a.tp[mat][e]);
+  const int k2 = a.k2[mat][e];
+  // a width the host should have refused, or not the one it promised
+  if (k2 < 2 || k2 > 16 || (a.k2_all == 8 && k2 != 8)) {
+    if (tid == 0) atomicCAS(&g_kernel_status, 0, ST_BAD_INDEX);
+    return;
+  }
+  if (warp == TC_MMA_WARP) tmem_alloc(flags, TC_TMEM_COLS);
+  if (tid < TC_PAIRS) pair_sh[tid] = tid < cnt ? ld_dep(members + first + tid) : -1;
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = flags[0];
+  const int nmma = cnt > 16 ? 32 : 16;
+  // the parts of K: `part` k-tiles of 16 inputs each, as grouped_kernel's warps take them (K / 16 is a multiple of 8)
+  const int steps = a.K / TC_STEP, part = (a.K / 16) / TC_PARTS;
+  const int stages = steps / 2;
+  const int sp_n = k2 <= 8 ? 8 : 4, stage_bytes = 2 * TC_STEP / 16 * (TC_COLS / 16) * 16 * k2;   // Ring<k2>
+  bool ok = true;
+
+  if (warp == TC_LOAD_WARP) {
+    // Trellis: a lane a row of tiles.  Inputs: lane -> 16-byte chunk c of pairs r0, r0 + 4, ..; pairs past the item's
+    // last are left as they are (an MMA column depends on its own pair only, and theirs are never stored).
+    constexpr int PER = TC_PAIRS / 4, LAG = 2;
+    const uint32_t row_bytes = (uint32_t)(TC_COLS / 16) * 16 * k2;
+    const size_t row_stride = (size_t)(a.N >> 4) * 16 * k2, stage_stride = (2 * TC_STEP / 16) * row_stride;
+    const uint8_t* src = T + (size_t)lane * row_stride + (size_t)blk * row_bytes;
+    const int c = lane & 7, r0 = lane >> 3;
+    const __half* xk = xin + c * 8;
+    uint32_t row[PER];                                // in 8 inputs
+#pragma unroll
+    for (int j = 0; j < PER; ++j) row[j] = (uint32_t)max(pair_sh[r0 + 4 * j], 0) * (uint32_t)(a.K >> 3);
+    int s = 0, ph = 1, back = 0, sp = 0, pph = 1;     // ph, pph: a ring's first round finds every stage free
+    constexpr int rows = 2 * TC_STEP / 16;            // K is a multiple of 128: whole stages
+    int p = 0;
+    for (; p < stages; ++p) {
+      if (p >= sp_n) ok = mbar_wait_warp(packed_free + sp, pph);
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(packed_full + sp, (uint32_t)rows * row_bytes);
+      __syncwarp();
+      if (lane < rows) bulk_g2s(smem + sp * stage_bytes + lane * row_bytes, src, row_bytes, packed_full + sp);
+      src += stage_stride;
+      if (++sp == sp_n) {
+        sp = 0;
+        pph ^= 1;
+      }
+      if (p >= SM::SB) ok = mbar_wait_warp(b_free + s, ph);
+      if (!ok) {
+        ++p;
+        break;
+      }
+      uint8_t* btile = smem + SM::B_OFFSET + s * (2 * SM::B_TILE) + r0 * 128;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        if (4 * j >= cnt) break;
+        const int r = r0 + 4 * j;
+        if (r < cnt) {
+          uint8_t* dst = btile + 4 * j * 128 + ((c ^ (r & 7)) << 4);
+          const __half* from = xk + (size_t)row[j] * 8;
+          cp_async16(dst, from);
+          cp_async16(dst + SM::B_TILE, from + TC_STEP);
+        }
+      }
+      xk += 2 * TC_STEP;
+      cp_async_commit();
+      if (++s == SM::SB) {
+        s = 0;
+        ph ^= 1;
+      }
+      if (p >= LAG) {                                 // the stage LAG back has landed: publish it
+        cp_async_wait<LAG>();
+        fence_async_smem();
+        mbar_arrive(b_ready + back);
+        if (++back == SM::SB) back = 0;
+      }
+    }
+    cp_async_wait<0>();
+    fence_async_smem();
+    if (ok)
+      for (int f = max(0, stages - LAG); f < stages; ++f) {
+        mbar_arrive(b_ready + back);
+        if (++back == SM::SB) back = 0;
+      }
+    else if (lane == 0)                                // give the trellis copies in flight a while to land
+      for (int f = max(0, p - sp_n); f < p; ++f) mbar_wait_for(packed_full + (f & (sp_n - 1)), (f / sp_n) & 1, 10000000ull);
+    __syncwarp();
+  } else if (warp == TC_MMA_WARP) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_f16(nmma);
+      const uint64_t desc0 = umma_desc(smem_addr(smem + SM::B_OFFSET));     // addresses count 16 bytes
+      int s = 0, ph = 0, done = 0;                    // k-tiles done of the part
+      uint32_t d = tmem;                              // its accumulator
+      for (int g = 0; g < steps; ++g) {
+        const int t = g & 1, set = g & (TC_SETS - 1);
+        if (t == 0) ok = mbar_wait(b_ready + s, ph);
+        ok = ok && mbar_wait(a_ready + set, (g / TC_SETS) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t at = tmem + TC_A_COL + set * 32;
+        const uint64_t desc = desc0 + (uint32_t)((2 * s + t) * (SM::B_TILE >> 4));
+#pragma unroll
+        for (int ks = 0; ks < TC_STEP / 16; ++ks) {
+          umma_ta(d, at + ks * 8, desc + ks * 2, idesc, done > 0 ? 1u : 0u);   // a part's first k-tile starts its accumulator
+          if (++done == part) {
+            done = 0;
+            d += TC_PAIRS;
+          }
+        }
+        umma_commit(a_free + set);
+        if (t == 1) {
+          umma_commit(b_free + s);
+          if (++s == SM::SB) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      if (ok) umma_commit(acc_ready);
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, set = warp >> 2;
+    const uint32_t a_dst = tmem + ((uint32_t)(32 * q) << 16) + TC_A_COL + set * 32;
+#define TFB_K2(K2_)                                                                                                    \
+  case K2_:                                                                                                            \
+    ok = decode_stages<CB, K2_>(smem, packed_full, packed_free, a_ready, a_free, a_dst, set, q, steps, lane);          \
+    break;
+    switch (k2) {
+      TFB_K2(2) TFB_K2(3) TFB_K2(4) TFB_K2(5) TFB_K2(6) TFB_K2(7) TFB_K2(8) TFB_K2(9) TFB_K2(10) TFB_K2(11) TFB_K2(12)
+      TFB_K2(13) TFB_K2(14) TFB_K2(15) TFB_K2(16)
+    }
+#undef TFB_K2
+    if (ok) ok = mbar_wait_warp(acc_ready, 0);
+  }
+  pdl_launch_dependents();
+  tc_fence_after();
+  bool good = !__syncthreads_or(ok ? 0 : 1);          // a wait ran out (recorded): store nothing
+  // The accumulators, the parts added in order, as [pair][column] in the ring's memory (every copy has landed and been
+  // read).  Warp -> lane quarter q (columns 32 q + lane) and 8 of the pairs.
+  float* acc_sh = reinterpret_cast<float*>(smem);
+  constexpr int EP = TC_PAIRS / TC_SETS;
+  const int q = warp & 3, j0 = (warp >> 2) * EP;
+  if (good && warp < TC_DEC_WARPS && j0 < cnt) {
+    float v[EP];
+    uint32_t r[EP];
+    const uint32_t from = tmem + ((uint32_t)(32 * q) << 16) + j0;
+    tmem_ld8(from, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < EP; ++j) v[j] = __uint_as_float(r[j]);
+    for (int i = 1; i < TC_PARTS; ++i) {
+      tmem_ld8(from + i * TC_PAIRS, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < EP; ++j) v[j] += __uint_as_float(r[j]);
+    }
+    float* z = a.z + (size_t)mat * a.P * a.N + blk * TC_COLS + 32 * q + lane;
+#pragma unroll
+    for (int j = 0; j < EP; ++j) {
+      if (j0 + j >= cnt) continue;
+      acc_sh[(j0 + j) * TC_COLS + 32 * q + lane] = v[j];
+      if (a.epi != GE_DOWN) z[(size_t)pair_sh[j0 + j] * a.N] = v[j];
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == TC_MMA_WARP) tmem_dealloc(tmem, TC_TMEM_COLS);
+  if (!good || a.epi == GE_NONE) return;
+  if (a.epi == GE_GATEUP) {
+    // whoever finishes last of the two matrices' CTAs finds the other's part of the block in z and runs the epilogue
+    int* counter = a.arrive + (size_t)it * (a.N >> 7) + blk;
+    if (tid == 0) {
+      const int seen = arrive_count(counter);
+      flags[1] = seen == a.mats - 1;
+      if (seen == a.mats - 1) *counter = 0;           // nobody else touches it before the next launch
+    }
+    __syncthreads();
+    if (!flags[1]) return;
+  }
+  // a half warp a pair (the transform's shuffles need every lane of the warp: a half without a pair repeats the warp's
+  // first pair and stores nothing); pairs fill an item from the front, so a warp whose first pair is missing is done
+  const int sub = lane & 15, half = lane >> 4;
+  for (int p0 = 2 * warp; p0 < cnt; p0 += 2 * (TC_THREADS / 32)) {
+    const bool have = p0 + half < cnt;
+    const int i = have ? p0 + half : p0, p = pair_sh[i];
+    const size_t at = (size_t)p * a.N + blk * TC_COLS, sc = (size_t)e * a.N + blk * TC_COLS;
+    float own[8];
+    load8_shared(acc_sh + i * TC_COLS + 8 * sub, own);
+    if (a.epi == GE_GATEUP) {
+      float other[8];
+      load8(a.z + (size_t)(1 - mat) * a.P * a.N + at + 8 * sub, other);
+      float(&g)[8] = mat == 0 ? own : other;
+      float(&u)[8] = mat == 0 ? other : own;
+      gateup_block(g, u, a.sv[0] + sc, a.sv[1] + sc, a.suh_next + sc, static_cast<__half*>(a.out) + at, sub, a.limit,
+                   a.act_mode, have);
+    } else {
+      down_block(own, a.sv[0] + sc, static_cast<float*>(a.out) + at, sub, have);
+    }
   }
 }
 
@@ -849,8 +1220,8 @@ extern "C" int tfb_exl3_prologue(const void* x, int64_t x_stride, int x_is_fp16,
   const exl3::WidthOrder wo = {{k2_g, k2_u, k2_d}, sorted, sorted_stride};
   TFB_REQUIRE((suh1 == nullptr) == (out1 == nullptr), "exl3_prologue: the second matrix's scales and output come together");
   TFB_REQUIRE(!sort || (members && items && counts && ucount), "exl3_prologue: null sort table");
-  TFB_REQUIRE(sort == 0 || sort == 8 * exl3::GR_PT || sort == 8 * exl3::GR_WIDE_PT,
-              "exl3_prologue: sort is 0 (the caller sorted), %d or %d (pairs an item)", 8 * exl3::GR_PT, 8 * exl3::GR_WIDE_PT);
+  TFB_REQUIRE(sort == 0 || sort == exl3::GR_PAIRS || sort == exl3::TC_PAIRS,
+              "exl3_prologue: sort is 0 (the caller sorted), %d or %d (pairs an item)", exl3::GR_PAIRS, exl3::TC_PAIRS);
   TFB_REQUIRE(K > 0 && K % 128 == 0, "exl3_prologue: K must be a multiple of 128");
   TFB_REQUIRE(slots >= 1 && slots <= 32 && x_stride >= K && x_stride % 8 == 0, "exl3_prologue: bad slots or stride");
   TFB_REQUIRE(aligned16(x) && aligned16(suh0) && aligned16(out0) && aligned16(suh1) && aligned16(out1),
@@ -882,7 +1253,7 @@ extern "C" int tfb_exl3_prologue(const void* x, int64_t x_stride, int x_is_fp16,
   return check_cuda(e, "exl3_prologue");
 }
 
-static int exl3_grouped_launch(const char* who, const exl3::GroupedArgs& a, int cb, int max_items, int item_pairs,
+static int exl3_grouped_launch(const char* who, exl3::GroupedArgs a, int cb, int max_items, int item_pairs,
                                int k2_all, int col_tiles, void* stream) {
   TFB_REQUIRE(col_tiles == exl3::GR_NTB || col_tiles == exl3::GR_NARROW_NTB, "%s: %d or %d column tiles a block, not %d",
               who, exl3::GR_NTB, exl3::GR_NARROW_NTB, col_tiles);
@@ -890,28 +1261,43 @@ static int exl3_grouped_launch(const char* who, const exl3::GroupedArgs& a, int 
               "%s: k2_all is 0, -1 (the widths differ) or the one width of every tensor", who);
   TFB_REQUIRE(k2_all == 8 || col_tiles == exl3::GR_NTB, "%s: only a launch of 4.00-bit tensors (k2_all 8) takes blocks of %d "
               "column tiles", who, exl3::GR_NARROW_NTB);
-  TFB_REQUIRE(item_pairs == 8 * exl3::GR_PT || item_pairs == 8 * exl3::GR_WIDE_PT, "%s: items of %d or %d pairs, not %d",
-              who, 8 * exl3::GR_PT, 8 * exl3::GR_WIDE_PT, item_pairs);
+  TFB_REQUIRE(item_pairs == exl3::GR_PAIRS || item_pairs == exl3::TC_PAIRS, "%s: items of %d or %d pairs, not %d",
+              who, exl3::GR_PAIRS, exl3::TC_PAIRS, item_pairs);
   TFB_REQUIRE(a.K > 0 && a.N > 0 && a.K % 128 == 0 && a.N % 128 == 0, "%s: K and N must be multiples of 128", who);
   TFB_REQUIRE(cb >= 0 && cb <= 2, "%s: codebook must be 0 (3inst), 1 (mcg) or 2 (mul1)", who);
   TFB_REQUIRE(max_items >= 0 && a.P >= 0, "%s: bad sizes", who);
   if (max_items == 0 || a.P == 0) return TFB_OK;
   TFB_REQUIRE(max_items <= 65535, "%s: too many items for one launch", who);
-  const dim3 grid(a.N / (16 * col_tiles), max_items, a.mats);          // an item's column blocks run together
   auto st = static_cast<cudaStream_t>(stream);
+  cudaError_t e;
+  if (item_pairs == exl3::TC_PAIRS) {
+    a.k2_all = k2_all == 8 ? 8 : 0;
+    using Kernel = void (*)(exl3::GroupedArgs);
+    const Kernel kern = cb == 0   ? Kernel(exl3::grouped_tc_kernel<0>)
+                        : cb == 1 ? Kernel(exl3::grouped_tc_kernel<1>)
+                                  : Kernel(exl3::grouped_tc_kernel<2>);
+    static bool configured[3][64] = {};
+    int dev = 0;
+    TFB_CUDA(cudaGetDevice(&dev), who);
+    if (dev < 0 || dev >= 64) return fail(TFB_ERR_ARG, "%s: device index %d out of range", who, dev);
+    if (!configured[cb][dev]) {
+      TFB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, exl3::TrellisSmem::TOTAL), who);
+      configured[cb][dev] = true;
+    }
+    return check_cuda(launch(kern, dim3(a.N / exl3::TC_COLS, max_items, a.mats), dim3(exl3::TC_THREADS),
+                             (size_t)exl3::TrellisSmem::TOTAL, st, a),
+                      who);
+  }
+  const dim3 grid(a.N / (16 * col_tiles), max_items, a.mats);          // an item's column blocks run together
   const dim3 block(exl3::GR_WARPS * 32);
-  const bool wide = item_pairs == 8 * exl3::GR_WIDE_PT;
   const bool four = k2_all == 8;                      // the one width with a kernel of its own (4.00 bits a weight)
   const bool narrow = col_tiles == exl3::GR_NARROW_NTB;
-  cudaError_t e;
-#define TFB_GR4(CB_, PT_, K2F_) launch(exl3::grouped_kernel<CB_, PT_, K2F_, exl3::GR_NTB, false>, grid, block, 0, st, a)
-#define TFB_GRN(CB_, PT_) launch(exl3::grouped_kernel<CB_, PT_, 8, exl3::GR_NARROW_NTB, false>, grid, block, 0, st, a)
-#define TFB_GRC(CB_, PT_) launch(exl3::grouped_kernel<CB_, PT_, 0, exl3::GR_NTB, true>, grid, block, 0, st, a)
-#define TFB_GR(CB_)                                                                                     \
-  e = k2_all == -1 ? (wide ? TFB_GRC(CB_, exl3::GR_WIDE_PT) : TFB_GRC(CB_, exl3::GR_PT))                 \
-      : narrow     ? (wide ? TFB_GRN(CB_, exl3::GR_WIDE_PT) : TFB_GRN(CB_, exl3::GR_PT))                 \
-      : four       ? (wide ? TFB_GR4(CB_, exl3::GR_WIDE_PT, 8) : TFB_GR4(CB_, exl3::GR_PT, 8))           \
-                   : (wide ? TFB_GR4(CB_, exl3::GR_WIDE_PT, 0) : TFB_GR4(CB_, exl3::GR_PT, 0))
+#define TFB_GR4(CB_, K2F_, NTB_, COMPACT_) launch(exl3::grouped_kernel<CB_, K2F_, NTB_, COMPACT_>, grid, block, 0, st, a)
+#define TFB_GR(CB_)                                                  \
+  e = k2_all == -1 ? TFB_GR4(CB_, 0, exl3::GR_NTB, true)             \
+      : narrow     ? TFB_GR4(CB_, 8, exl3::GR_NARROW_NTB, false)     \
+      : four       ? TFB_GR4(CB_, 8, exl3::GR_NTB, false)            \
+                   : TFB_GR4(CB_, 0, exl3::GR_NTB, false)
   if (cb == 0) {
     TFB_GR(0);
   } else if (cb == 1) {
@@ -919,10 +1305,8 @@ static int exl3_grouped_launch(const char* who, const exl3::GroupedArgs& a, int 
   } else {
     TFB_GR(2);
   }
-#undef TFB_GRC
-#undef TFB_GRN
-#undef TFB_GR4
 #undef TFB_GR
+#undef TFB_GR4
   return check_cuda(e, who);
 }
 

@@ -25,7 +25,7 @@ ACT_BF16, ACT_F32 = 0, 1          # SwiGLU with the GLM family's bf16 roundings 
 K2_SUPPORTED = tuple(range(2, 17))   # half-bits a value: 1..8 bits and every half-integer rate between
 LAUNCHES_PER_CALL = 4             # kernels one ``routed`` call with weights enqueues (3 without)
 ITEM_PAIRS = 16                   # pairs an item of the sort holds: two mma tiles share one decoded weight tile
-WIDE_ITEM_PAIRS = 32              # the same with four mma tiles, for calls with many pairs an expert
+WIDE_ITEM_PAIRS = 32              # the same for the kernel's tensor-memory form, for calls with many pairs an expert
 WIDE_FROM = 12                    # pairs an expert on average from which a call sorts into the wide items
 
 # (16-column tiles a block, K-slice warps, K splits across blocks, tiles in flight): this library's one setting.

@@ -329,3 +329,30 @@ def test_the_short_loop_build_for_mixed_widths_gives_the_same_bits(R, monkeypatc
     torch.cuda.synchronize()
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     assert bool(torch.isfinite(outs[0][0]).all()) and float(outs[0][0].abs().max()) > 0
+
+
+@pytest.mark.parametrize("cb, widths", [(0, (8, 8, 8)), (1, (16, 3, 9)), (2, (2, 7, 12)), (0, (5, 6, 4)), (1, (10, 11, 13)),
+                                        (2, (14, 15, 8))])
+@pytest.mark.parametrize("dims, width", [(128, 128), (256, 384), (640, 256)])
+def test_wide_items_give_the_narrow_items_bits(cb, widths, dims, width, monkeypatch):
+    """The tensor-memory kernel (items of up to 32 pairs) against the register kernel (16), bit for bit: one to 97 pairs an
+    expert, inputs whose four parts do not fall on whole steps (128, 384, 640), every width of the format."""
+
+    from tensorfold_b200 import _lib
+    from tensorfold_b200.exl3 import experts
+
+    counts = [1, 2, 15, 16, 17, 31, 32, 33, 97]
+    ex, _ = _layer(len(counts), dims, width, [widths if e % 2 else widths[::-1] for e in range(len(counts))], cb, 3)
+    g = torch.Generator().manual_seed(4)
+    pick = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)])
+    pick = pick[torch.randperm(pick.numel(), generator=g)].unsqueeze(1).to(DEV).contiguous()
+    rows = pick.shape[0]
+    x = torch.randn((rows, dims), generator=g).to(torch.bfloat16).to(DEV)
+    got = {}
+    for per in (experts.ITEM_PAIRS, experts.WIDE_ITEM_PAIRS):
+        monkeypatch.setattr(experts, "item_pairs", lambda pairs, count: per)
+        s = experts.Scratch(ex, rows, 1)
+        got[per] = experts.routed(x, pick, None, ex, s, None, rows).clone()
+        torch.cuda.synchronize()
+        assert _lib.kernel_status() == 0 and int(s.arrive.abs().max()) == 0
+    assert torch.isfinite(got[16]).all() and torch.equal(got[16], got[32])
