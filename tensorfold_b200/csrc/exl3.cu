@@ -371,7 +371,10 @@ __device__ __forceinline__ bool decode_stages(const uint8_t* ring, uint64_t* pac
 
 // ---- 128-point Walsh-Hadamard transform by 16 lanes, 8 consecutive values a lane ---------------------------------
 // Strides 1, 2, 4 inside the lane, 8 .. 64 across the 16 lanes of a half warp (sub = lane % 16); a warp transforms two
-// blocks at once.  Not scaled.
+// blocks at once.  Not scaled.  FMA: o + v or o - v across the lanes as one fma with the lane's sign (the product is exact:
+// the same bits) instead of two adds and a select - for the kernels that do little else (the prologue at 512 tokens of a
+// 4096-wide layer 43 -> 38 us); inside grouped_kernel the extra live values cost its main loop 5 %.
+template <bool FMA>
 __device__ __forceinline__ void hadamard128(float (&v)[8], int sub) {
 #pragma unroll
   for (int h = 1; h < 8; h <<= 1)
@@ -383,12 +386,37 @@ __device__ __forceinline__ void hadamard128(float (&v)[8], int sub) {
         v[i + h] = a - b;
       }
 #pragma unroll
-  for (int m = 1; m < 16; m <<= 1)
+  for (int m = 1; m < 16; m <<= 1) {
+    const float sign = (sub & m) ? -1.f : 1.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float o = __shfl_xor_sync(0xffffffffu, v[i], m);
-      v[i] = (sub & m) ? o - v[i] : v[i] + o;
+      if constexpr (FMA)
+        v[i] = fmaf(sign, v[i], o);
+      else
+        v[i] = (sub & m) ? o - v[i] : v[i] + o;
     }
+  }
+}
+
+// The same by 8 lanes, 16 consecutive values a lane (a warp transforms four blocks at once): a quarter fewer shuffles a
+// block, and the strides in the same order, so the same bits.
+__device__ __forceinline__ void hadamard128_wide(float (&v)[16], int sub) {
+#pragma unroll
+  for (int h = 1; h < 16; h <<= 1)
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if ((i & h) == 0) {
+        const float a = v[i], b = v[i + h];
+        v[i] = a + b;
+        v[i + h] = a - b;
+      }
+#pragma unroll
+  for (int m = 1; m < 8; m <<= 1) {
+    const float sign = (sub & m) ? -1.f : 1.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = fmaf(sign, v[i], __shfl_xor_sync(0xffffffffu, v[i], m));
+  }
 }
 
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
@@ -432,8 +460,8 @@ __device__ __forceinline__ void gateup_block(float (&g)[8], float (&u)[8], const
   load8(svh_g + 8 * sub, sg);
   load8(svh_u + 8 * sub, su);
   load8(suh_d + 8 * sub, sd);
-  hadamard128(g, sub);
-  hadamard128(u, sub);
+  hadamard128<false>(g, sub);
+  hadamard128<false>(u, sub);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     float act;
@@ -448,7 +476,7 @@ __device__ __forceinline__ void gateup_block(float (&g)[8], float (&u)[8], const
     }
     g[i] = act * sd[i];
   }
-  hadamard128(g, sub);
+  hadamard128<false>(g, sub);
   if (store) store8(xd + 8 * sub, g, HAD_SCALE);
 }
 
@@ -456,7 +484,7 @@ __device__ __forceinline__ void gateup_block(float (&g)[8], float (&u)[8], const
 __device__ __forceinline__ void down_block(float (&v)[8], const __half* svh, float* y, int sub, bool store) {
   float s[8];
   load8(svh + 8 * sub, s);
-  hadamard128(v, sub);
+  hadamard128<false>(v, sub);
   if (!store) return;
   float4 a, b;
   a.x = v[0] * HAD_SCALE * s[0]; a.y = v[1] * HAD_SCALE * s[1]; a.z = v[2] * HAD_SCALE * s[2]; a.w = v[3] * HAD_SCALE * s[3];
@@ -912,20 +940,54 @@ grouped_tc_kernel(const GroupedArgs a) {
 namespace tfb {
 namespace exl3 {
 
-// W_q [K, N] fp16 of one matrix through the same lane decode (the bit-exactness hook).
+// W_q [K, N] fp16 of one matrix through the same lane decode (the bit-exactness hook, and the prompt form's weights).  A
+// warp takes a row of eight tiles: all their words in flight, decoded, transposed through shared memory (the fragments hold
+// pairs of inputs, the rows want pairs of columns) and stored as whole rows of 256 bytes.  vec: out is 16-byte aligned.
+// Bound by the write of W_q; with one tile a block and 2-byte stores a 4096 x 4096 matrix
+// at 4.00 bits took 35 us, this one 8.3 (42 MB: 5.0 TB/s).
+constexpr int DQ_WARPS = 8, DQ_TILES = 8, DQ_STRIDE = 16 * DQ_TILES + 8;   // halves a staged row: rows 16 bytes apart mod 128
+
 template <int CB, int K2>
-__global__ void dequant_kernel(const uint32_t* __restrict__ T, __half* __restrict__ out, int K, int N) {
-  const int kt = blockIdx.x, nt = blockIdx.y, lane = threadIdx.x, g = lane >> 2, t = lane & 3;
-  uint32_t w[Win<K2>::NW], a[4];
-  lane_words<K2, true>(T + ((size_t)kt * (N >> 4) + nt) * Win<K2>::TW, lane, w);
-  decode_words<CB, K2>(w, lane, a);
-  // a0 = (col g, k 2t, 2t+1), a1 = (col g + 8, ...), a2 = (col g, k 2t + 8, ..), a3 = (col g + 8, k 2t + 8, ..)
+__global__ void __launch_bounds__(DQ_WARPS * 32)
+dequant_kernel(const uint32_t* __restrict__ T, __half* __restrict__ out, int K, int N, int vec) {
+  constexpr int NW = Win<K2>::NW;
+  __shared__ __align__(16) __half rows[DQ_WARPS][16 * DQ_STRIDE];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ntiles = N >> 4, nblk = (ntiles + DQ_TILES - 1) / DQ_TILES;
+  const int64_t u = (int64_t)blockIdx.x * DQ_WARPS + warp;
+  const int kt = (int)(u / nblk), nt0 = (int)(u - (int64_t)kt * nblk) * DQ_TILES;
+  pdl_wait();
+  after_wait(T);
+  if (kt >= (K >> 4)) return;
+  const int live = min(DQ_TILES, ntiles - nt0);
+  const uint32_t* src = T + ((size_t)kt * ntiles + nt0) * Win<K2>::TW;
+  uint32_t w[DQ_TILES][NW];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const __half2 h = *reinterpret_cast<const __half2*>(&a[q]);
-    const int col = nt * 16 + g + 8 * (q & 1), row = kt * 16 + 2 * t + 8 * (q >> 1);
-    out[(size_t)row * N + col] = __low2half(h);
-    out[(size_t)(row + 1) * N + col] = __high2half(h);
+  for (int i = 0; i < DQ_TILES; ++i) lane_words<K2, true>(src + (size_t)(i < live ? i : 0) * Win<K2>::TW, lane, w[i]);
+  __half* stage = rows[warp];
+  // the transposing store: lane 8 m + r gives the address of input row r of matrix m = (columns 8 (m & 1), inputs 8 (m >> 1))
+  const uint32_t to = smem_addr(stage + ((lane >> 4) * 8 + (lane & 7)) * DQ_STRIDE + ((lane >> 3) & 1) * 8);
+#pragma unroll
+  for (int i = 0; i < DQ_TILES; ++i) {
+    uint32_t a[4];
+    decode_words<CB, K2>(w[i], lane, a);
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};\n" ::"r"(to + i * 32), "r"(a[0]),
+                 "r"(a[1]), "r"(a[2]), "r"(a[3])
+                 : "memory");
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int row = 2 * r + (lane >> 4), c = (lane & 15) * 8;
+    if (c >= live * 16) continue;
+    const uint4 v = *reinterpret_cast<const uint4*>(stage + row * DQ_STRIDE + c);
+    __half* dst = out + (size_t)(kt * 16 + row) * N + nt0 * 16 + c;
+    if (vec) {
+      *reinterpret_cast<uint4*>(dst) = v;
+    } else {
+      const __half* h = reinterpret_cast<const __half*>(&v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dst[j] = h[j];
+    }
   }
 }
 
@@ -1002,17 +1064,18 @@ exl3_prologue_kernel(const int* __restrict__ picks, int P, int E, int slots, int
     const int e = picks[p];
     const bool routed = have && e >= 0 && e < E;
     const int es = routed ? e : 0;
-    float xv[8];
+    float xv[8], s[2][8];
     exl3::load8(x + (size_t)(p / slots) * x_stride + blk * 128 + 8 * sub, xv);
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const __half* suh = m ? suh1 : suh0;
-      if (suh == nullptr) continue;
-      float s[8], v[8];
-      exl3::load8(suh + (size_t)es * K + blk * 128 + 8 * sub, s);
+    for (int m = 0; m < 2; ++m)
+      if ((m ? suh1 : suh0) != nullptr) exl3::load8((m ? suh1 : suh0) + (size_t)es * K + blk * 128 + 8 * sub, s[m]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = xv[i] * s[i];
-      exl3::hadamard128(v, sub);
+    for (int m = 0; m < 2; ++m) {
+      if ((m ? suh1 : suh0) == nullptr) continue;
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = xv[i] * s[m][i];
+      exl3::hadamard128<true>(v, sub);
       if (routed) exl3::store8((m ? out1 : out0) + (size_t)p * K + blk * 128 + 8 * sub, v, exl3::HAD_SCALE);
     }
   }
@@ -1020,39 +1083,53 @@ exl3_prologue_kernel(const int* __restrict__ picks, int P, int E, int slots, int
 }
 
 // The prompt form's epilogue: out[m, block] = rotate(z[m, block]) / sqrt(128) * svh + bias for every row and
-// 128-column block of a product z [M, N] fp32, a half warp a block.
+// 128-column block of a product z [M, N] fp32, eight lanes a block.  vec: the rows of out are 16-byte aligned.
 // (the epilogue of src/tensorfold/cuda/exl3/prefill.py:15-44 `_gemm`)
 template <typename TOUT>
 __global__ void __launch_bounds__(256)
 exl3_rot_out_kernel(const float* __restrict__ z, const __half* __restrict__ svh, const __half* __restrict__ bias,
-                    TOUT* __restrict__ out, int64_t out_stride, int M, int N) {
-  const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
+                    TOUT* __restrict__ out, int64_t out_stride, int M, int N, int vec) {
+  const int lane = threadIdx.x & 31, sub = lane & 7, quad = lane >> 3;
   const int nblk = N >> 7;
   const int64_t units = (int64_t)M * nblk;
   const int64_t warps = (int64_t)gridDim.x * 8;
   pdl_wait();
   after_wait(z);
-  for (int64_t u0 = 2 * ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)); u0 < units; u0 += 2 * warps) {
-    const bool have = u0 + half < units;              // the transform's shuffles need every lane: an idle half repeats u0
-    const int64_t u = have ? u0 + half : u0;
+  for (int64_t u0 = 4 * ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)); u0 < units; u0 += 4 * warps) {
+    const bool have = u0 + quad < units;              // the transform's shuffles need every lane: an idle one repeats u0
+    const int64_t u = have ? u0 + quad : u0;
     const int m = (int)(u / nblk), blk = (int)(u - (int64_t)m * nblk);
-    float v[8], s[8], b[8];
-    const float4* src = reinterpret_cast<const float4*>(z + (size_t)m * N + blk * 128 + 8 * sub);
-    const float4 lo = src[0], hi = src[1];
-    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-    exl3::load8(svh + blk * 128 + 8 * sub, s);
+    float v[16], s[2][8], b[2][8];
+    const float4* src = reinterpret_cast<const float4*>(z + (size_t)m * N + blk * 128 + 16 * sub);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) b[i] = 0.f;
-    if (bias != nullptr) exl3::load8(bias + blk * 128 + 8 * sub, b);
-    exl3::hadamard128(v, sub);
+    for (int i = 0; i < 4; ++i) {
+      const float4 t = src[i];
+      v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      exl3::load8(svh + blk * 128 + 16 * sub + 8 * h, s[h]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) b[h][i] = 0.f;
+      if (bias != nullptr) exl3::load8(bias + blk * 128 + 16 * sub + 8 * h, b[h]);
+    }
+    exl3::hadamard128_wide(v, sub);
     if (!have) continue;
-    TOUT* dst = out + (size_t)m * out_stride + blk * 128 + 8 * sub;
+    __align__(16) TOUT y[16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float y = fmaf(v[i] * exl3::HAD_SCALE, s[i], b[i]);
-      if constexpr (sizeof(TOUT) == 4) dst[i] = y;
-      else if constexpr (std::is_same<TOUT, __half>::value) dst[i] = __float2half_rn(y);
-      else dst[i] = __float2bfloat16_rn(y);
+    for (int i = 0; i < 16; ++i) {
+      const float f = fmaf(v[i] * exl3::HAD_SCALE, s[i >> 3][i & 7], b[i >> 3][i & 7]);
+      if constexpr (sizeof(TOUT) == 4) y[i] = f;
+      else if constexpr (std::is_same<TOUT, __half>::value) y[i] = __float2half_rn(f);
+      else y[i] = __float2bfloat16_rn(f);
+    }
+    TOUT* dst = out + (size_t)m * out_stride + blk * 128 + 16 * sub;
+    if (vec) {
+#pragma unroll
+      for (int i = 0; i < (int)sizeof(TOUT); ++i) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(y)[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) dst[i] = y[i];
     }
   }
   pdl_launch_dependents();
@@ -1104,13 +1181,18 @@ extern "C" int tfb_exl3_dequant(const void* trellis, void* out, int K, int N, in
   TFB_REQUIRE(K > 0 && N > 0 && K % 16 == 0 && N % 16 == 0, "exl3_dequant: K and N must be multiples of 16");
   TFB_REQUIRE(cb >= 0 && cb <= 2, "exl3_dequant: codebook must be 0 (3inst), 1 (mcg) or 2 (mul1)");
   if (int rc = exl3_check_k2("exl3_dequant", k2)) return rc;
-  const dim3 grid(K / 16, N / 16);
+  const int64_t warps = (int64_t)(K / 16) * ((N / 16 + exl3::DQ_TILES - 1) / exl3::DQ_TILES);
+  const int64_t blocks = (warps + exl3::DQ_WARPS - 1) / exl3::DQ_WARPS;
+  TFB_REQUIRE(blocks < (int64_t(1) << 31), "exl3_dequant: too many tiles");
+  const dim3 grid((unsigned)blocks);
   auto st = static_cast<cudaStream_t>(stream);
   auto* t = static_cast<const uint32_t*>(trellis);
   auto* o = static_cast<__half*>(out);
+  const int vec = aligned16(out) ? 1 : 0;             // rows are multiples of 32 bytes
+  cudaError_t e = cudaSuccess;
 #define TFB_DQ(CB_, K2_)                                               \
   case K2_:                                                            \
-    exl3::dequant_kernel<CB_, K2_><<<grid, 32, 0, st>>>(t, o, K, N);   \
+    e = launch(exl3::dequant_kernel<CB_, K2_>, grid, dim3(exl3::DQ_WARPS * 32), 0, st, t, o, K, N, vec); \
     break;
 #define TFB_DQ_ALL(CB_)                                                                                          \
   switch (k2) {                                                                                                  \
@@ -1121,7 +1203,7 @@ extern "C" int tfb_exl3_dequant(const void* trellis, void* out, int K, int N, in
   if (cb == 0) { TFB_DQ_ALL(0) } else if (cb == 1) { TFB_DQ_ALL(1) } else { TFB_DQ_ALL(2) }
 #undef TFB_DQ_ALL
 #undef TFB_DQ
-  return check_launch("exl3_dequant");
+  return check_cuda(e, "exl3_dequant");
 }
 
 // Opts a plan-sized kernel into the dynamic shared memory of PLAN_EMAX experts, once a device.
@@ -1413,18 +1495,20 @@ extern "C" int tfb_exl3_rot_out(const float* z, const void* svh, const void* bia
   TFB_REQUIRE(aligned16(z) && aligned16(svh) && aligned16(bias), "exl3_rot_out: 16-byte aligned rows");
   if (M <= 0) return TFB_OK;
   const int64_t units = (int64_t)M * (N / 128);
-  const int64_t want = (units + 15) / 16;
-  const dim3 grid((unsigned)(want < 8 * sm_count() ? want : 8 * sm_count()));
+  const int64_t want = (units + 31) / 32;
+  const dim3 grid((unsigned)(want < 16 * sm_count() ? want : 16 * sm_count()));
   auto st = static_cast<cudaStream_t>(stream);
   auto* sv = static_cast<const __half*>(svh);
   auto* bi = static_cast<const __half*>(bias);
+  const int vec = aligned16(out) && (out_stride * (out_type == 0 ? 4 : 2)) % 16 == 0 ? 1 : 0;
   cudaError_t e;
   if (out_type == 0)
-    e = launch(exl3_rot_out_kernel<float>, grid, dim3(256), 0, st, z, sv, bi, static_cast<float*>(out), out_stride, M, N);
+    e = launch(exl3_rot_out_kernel<float>, grid, dim3(256), 0, st, z, sv, bi, static_cast<float*>(out), out_stride, M, N, vec);
   else if (out_type == 1)
-    e = launch(exl3_rot_out_kernel<__half>, grid, dim3(256), 0, st, z, sv, bi, static_cast<__half*>(out), out_stride, M, N);
+    e = launch(exl3_rot_out_kernel<__half>, grid, dim3(256), 0, st, z, sv, bi, static_cast<__half*>(out), out_stride, M, N,
+               vec);
   else
     e = launch(exl3_rot_out_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, z, sv, bi, static_cast<__nv_bfloat16*>(out),
-               out_stride, M, N);
+               out_stride, M, N, vec);
   return check_cuda(e, "exl3_rot_out");
 }

@@ -356,3 +356,43 @@ def test_wide_items_give_the_narrow_items_bits(cb, widths, dims, width, monkeypa
         torch.cuda.synchronize()
         assert _lib.kernel_status() == 0 and int(s.arrive.abs().max()) == 0
     assert torch.isfinite(got[16]).all() and torch.equal(got[16], got[32])
+
+
+@pytest.mark.parametrize("n", [16, 112, 128, 144, 272])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_dequant_rows_of_any_width_and_alignment(n, offset):
+    """W_q by rows of eight tiles: fewer, exactly and more than eight column tiles, into memory that is 16-byte aligned or
+    only 2-byte aligned; bit for bit, and nothing outside the matrix is touched."""
+
+    from oracle import exl3 as ref
+    from tensorfold_b200 import _lib
+    from tensorfold_b200.exl3 import experts
+
+    for k2 in (2, 8, 11, 16):
+        t = _trellis(32, n, k2, torch.Generator().manual_seed(n + k2))
+        flat = torch.full((offset + 32 * n + 8,), 7.0, dtype=torch.float16, device=DEV)
+        _lib.call("tfb_exl3_dequant", t.data_ptr(), flat.data_ptr() + 2 * offset, 32, n, k2, 0,
+                  torch.cuda.current_stream().cuda_stream)
+        want = ref.unpack(t.cpu().numpy(), 0)
+        got = flat[offset:offset + 32 * n].view(32, n).cpu().numpy()
+        assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
+        assert (flat[:offset] == 7.0).all() and (flat[offset + 32 * n:] == 7.0).all()
+        assert np.array_equal(experts.dequant(t, 0).cpu().numpy().view(np.uint16), want.view(np.uint16))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows", [1, 3, 129])
+def test_prompt_matmul_into_unaligned_rows(rows, dtype):
+    """Rows of out that no 16-byte store fits (odd offset, odd stride) hold the same bits as aligned rows."""
+
+    from tensorfold_b200.exl3 import prefill
+    from tensorfold_b200.exl3.linear import Exl3Linear
+
+    g = torch.Generator().manual_seed(rows)
+    layer = Exl3Linear.from_tensors(_trellis(256, 384, 8, g), _scale(256, 1 / 16, g), _scale(384, 1.0, g), "3inst")
+    x = torch.randn((rows, 256), generator=g).to(torch.bfloat16).to(DEV)
+    ws = prefill.Workspace()
+    want = prefill.matmul(layer, x, torch.empty((rows, 384), dtype=dtype, device=DEV), ws)
+    wide = torch.full((rows, 387), 7.0, dtype=dtype, device=DEV)
+    prefill.matmul(layer, x, wide[:, 1:385], ws)
+    assert torch.equal(wide[:, 1:385], want) and (wide[:, 0] == 7.0).all() and (wide[:, 385:] == 7.0).all()
