@@ -2,14 +2,20 @@
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from ctypes import c_char_p, c_float, c_int, c_int64, c_void_p
 from functools import lru_cache
 from pathlib import Path
 
+import torch
+
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libtfb200.so"
 
 ERR_ARG, ERR_CUDA, ERR_DEVICE = -1, -2, -3
+
+# torch's own lookup of a device's current stream handle (what its compiled launchers call), where this build has it
+_RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 P, I, L, F = c_void_p, c_int, c_int64, c_float
 
@@ -94,6 +100,24 @@ def call(name: str, *args) -> None:
     if rc == ERR_ARG:
         raise ValueError(text)
     raise RuntimeError(text)
+
+
+_HERE = contextlib.nullcontext()
+
+
+def on(device):
+    """``with on(device):`` makes ``device`` current for a launch.  Entering torch's own context costs a few microseconds
+    of host time each call, more than a small launch takes on the device, and nearly every call is already there."""
+
+    return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+def stream(device) -> int:
+    """The handle of ``device``'s current stream."""
+
+    if _RAW_STREAM is not None and device.index is not None:
+        return _RAW_STREAM(device.index)                            # without a Stream object around it
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def kernel_status(stream: int = 0) -> int:

@@ -35,7 +35,7 @@ _CODEBOOKS = {"3inst": CB_3INST, "mcg": CB_MCG, "mul1": CB_MUL1}
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.stream(t.device)
 
 
 def codebook_id(name: str) -> int:
@@ -234,7 +234,7 @@ def group(pick: torch.Tensor, s: Scratch, R: int, experts: int) -> None:
     ``routed(..., group_first=False)`` finds its pairs grouped."""
 
     ids, members = s.window(R)
-    with torch.cuda.device(pick.device):
+    with _lib.on(pick.device):
         _lib.call("tfb_exl3_group", pick.data_ptr(), ids.data_ptr(), s.count.data_ptr(), members.data_ptr(),
                   s.tmp_members.data_ptr(), s.tmp_items.data_ptr(), s.tmp_counts.data_ptr(), R, s.slots, experts,
                   ids.shape[0], R, _stream(pick))
@@ -275,7 +275,7 @@ def routed(x: torch.Tensor, pick: torch.Tensor, wts: torch.Tensor | None, ex: Ex
     k2_gu, k2_d = width_of(ex.k2_gu, width, 2), width_of(ex.k2_d, dims, 1)
     # a layer of mixed widths: the prologue lays the items out width by width, once a projection
     order = [s.by_width[m].data_ptr() for m in range(3)] if ex.mixed and group_first else [0, 0, 0]
-    with torch.cuda.device(x.device):
+    with _lib.on(x.device):
         _lib.call("tfb_exl3_prologue", x.data_ptr(), x.stride(0), int(x.dtype == torch.float16), pick.data_ptr(),
                   ex.suh_g.data_ptr(), ex.suh_u.data_ptr(), s.xg.data_ptr(), s.xu.data_ptr(), R, dims, slots, ex.count,
                   per_item if group_first else 0, *sort, s.count.data_ptr(), ex.gate_k2.data_ptr(), ex.up_k2.data_ptr(),
@@ -307,7 +307,7 @@ def dequant(trellis: torch.Tensor, codebook: int | str) -> torch.Tensor:
     rows, cols = trellis.shape[0] * 16, trellis.shape[1] * 16
     words = trellis.contiguous()
     w_q = torch.empty((rows, cols), dtype=torch.float16, device=trellis.device)
-    with torch.cuda.device(trellis.device):
+    with _lib.on(trellis.device):
         _lib.call("tfb_exl3_dequant", words.data_ptr(), w_q.data_ptr(), rows, cols, k2_of(trellis), cb,
                   _stream(trellis))
     return w_q

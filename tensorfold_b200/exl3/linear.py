@@ -29,7 +29,7 @@ def k2_of(bits: float) -> int:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.stream(t.device)
 
 
 @dataclass
@@ -122,7 +122,7 @@ class Exl3Linear:
             z = torch.empty((m, self.n), dtype=torch.float32, device=dev)
         y = torch.empty((m, self.n), dtype=torch.float32, device=dev)
         s = _stream(x)
-        with torch.cuda.device(dev):
+        with _lib.on(dev):
             _lib.call("tfb_exl3_prologue", x.data_ptr(), x.stride(0), int(x.dtype == torch.float16),
                       t["pick"].data_ptr(), self.suh.data_ptr(), 0, xh.data_ptr(), 0, m, self.k, 1, 1, 0, 0, 0, 0, 0,
                       0, 0, 0, 0, 0, s)

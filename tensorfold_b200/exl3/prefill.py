@@ -61,12 +61,12 @@ def matmul(layer: Exl3Linear, x: torch.Tensor, out: torch.Tensor, ws: Workspace)
         return out
     x = x.contiguous()
     dev = x.device
-    st = torch.cuda.current_stream(dev).cuda_stream
+    st = _lib.stream(dev)
     xh = ws._grow("xh", m * k, torch.float16, dev)[:m * k].view(m, k)
     wq = ws._grow("w", k * n, torch.float16, dev)[:k * n].view(k, n)
     z = ws._grow("z", m * n, torch.float32, dev)[:m * n].view(m, n)
     pick = ws._grow("pick", m, torch.int32, dev)[:m]                # every row is a pair of the one "expert"
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         pick.zero_()
         _lib.call("tfb_exl3_prologue", x.data_ptr(), x.stride(0), int(x.dtype == torch.float16), pick.data_ptr(),
                   layer.suh.data_ptr(), 0, xh.data_ptr(), 0, m, k, 1, 1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, st)

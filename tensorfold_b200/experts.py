@@ -26,7 +26,7 @@ _SB = {torch.bfloat16: 0, torch.float16: 1}
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.stream(t.device)
 
 
 def _need_cuda(t: torch.Tensor, name: str) -> None:
@@ -50,7 +50,7 @@ def pack(words: torch.Tensor, scales: torch.Tensor, biases: torch.Tensor, gs: in
         raise ValueError("scales and biases must share a 2-byte dtype")
     out = torch.empty((e, n // COLS, k // gs, BLOCK), dtype=torch.int32, device=words.device)
     w, s, b = words.contiguous(), scales.contiguous(), biases.contiguous()
-    with torch.cuda.device(words.device):
+    with _lib.on(words.device):
         _lib.call("tfb_pack", w.data_ptr(), s.data_ptr(), b.data_ptr(), gs, out.data_ptr(), e, n, k, _stream(words))
     return out
 
@@ -67,7 +67,7 @@ def unpack(blocks: torch.Tensor, gs: int, dtype: torch.dtype = torch.bfloat16):
     words = torch.empty((e, n, k // 8), dtype=torch.int32, device=blocks.device)
     scales = torch.empty((e, n, kg), dtype=dtype, device=blocks.device)
     biases = torch.empty_like(scales)
-    with torch.cuda.device(blocks.device):
+    with _lib.on(blocks.device):
         _lib.call("tfb_unpack", blocks.data_ptr(), gs, words.data_ptr(), scales.data_ptr(), biases.data_ptr(), e, n, k,
                   _stream(blocks))
     return words, scales, biases
@@ -83,7 +83,7 @@ def dequantize(blocks: torch.Tensor, gs: int, *, prefill: bool = False,
     n, k = nb * COLS, kg * gs
     blocks = blocks.contiguous()
     out = torch.empty((e, n, k), dtype=torch.bfloat16 if prefill else torch.float32, device=blocks.device)
-    with torch.cuda.device(blocks.device):
+    with _lib.on(blocks.device):
         _lib.call("tfb_dequant", blocks.data_ptr(), gs, _SB[scale_dtype], 1 if prefill else 0, out.data_ptr(), e, n, k,
                   _stream(blocks))
     return out
@@ -182,7 +182,7 @@ def route(picks: torch.Tensor, plan: Plan, tile: int = PREFILL_TILE) -> None:
     plan.tile = tile if plan.prefill else plan.decode_tile
     if plan.tile < TILE:
         raise ValueError(f"items hold at least {TILE} pairs")
-    with torch.cuda.device(picks.device):
+    with _lib.on(picks.device):
         _lib.call("tfb_plan", picks.data_ptr(), rows * slots, plan.experts, plan.tile, plan.members.data_ptr(),
                   plan.items.data_ptr(), plan.counts.data_ptr(), _stream(picks))
 
@@ -198,7 +198,7 @@ def route_split(picks: torch.Tensor, plan: Plan, lo: int = 0) -> None:
         raise ValueError(f"picks {tuple(picks.shape)} do not fit a plan of {plan.rows} x {plan.slots}")
     _need_cuda(picks, "picks")
     plan.tile = plan.decode_tile
-    with torch.cuda.device(picks.device):
+    with _lib.on(picks.device):
         _lib.call("tfb_plan_split", picks.data_ptr(), rows * slots, lo, plan.experts, plan.tile, PREFILL_TILE, plan.hot,
                   plan.members.data_ptr(), plan.items.data_ptr(), plan.counts.data_ptr(), plan.big_items.data_ptr(),
                   plan.big_counts.data_ptr(), _stream(picks))
@@ -258,7 +258,7 @@ def _run(epi: int, x: torch.Tensor, slots: int, w: torch.Tensor, kg: int, nb: in
         raise ValueError("out: contiguous rows of n columns of the epilogue's dtype")
     if not w.is_contiguous():
         raise ValueError("w must be contiguous")
-    with torch.cuda.device(x.device):
+    with _lib.on(x.device):
         if prefill:
             _lib.call("tfb_experts_prefill", ex.gs, epi, x.data_ptr(), x.stride(0), slots, w.data_ptr(), kg, nb,
                       plan.items.data_ptr(), plan.counts.data_ptr(), plan.members.data_ptr(), out.data_ptr(), n,
@@ -320,7 +320,7 @@ def down_combine(act: torch.Tensor, ex: Experts, plan: Plan, y: torch.Tensor, ro
     if not ex.down.is_contiguous():
         raise ValueError("w must be contiguous")
     items = max_items(rows * plan.slots, plan.experts, plan.tile)
-    with torch.cuda.device(act.device):
+    with _lib.on(act.device):
         _lib.call("tfb_experts_down_combine", ex.gs, act.data_ptr(), act.stride(0), ex.down.data_ptr(),
                   ex.width // ex.gs, nb, plan.items.data_ptr(), plan.counts.data_ptr(), plan.members.data_ptr(),
                   y.data_ptr(), ex.dims, items * nb, _SB[ex.scale_dtype], plan.tile, wts.data_ptr(), plan.slots,

@@ -17,7 +17,7 @@ from . import experts as grouped
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.stream(t.device)
 
 
 def router(x: torch.Tensor, rows: torch.Tensor, out: torch.Tensor | None = None, *, prompt: bool = False) -> torch.Tensor:
@@ -37,7 +37,7 @@ def router(x: torch.Tensor, rows: torch.Tensor, out: torch.Tensor | None = None,
         out = torch.empty((m, ne), dtype=torch.float32, device=x.device)
     elif out.shape != (m, ne) or out.dtype != torch.float32 or not out.is_contiguous():
         raise ValueError("router: out must be contiguous fp32 [R, NE]")
-    with torch.cuda.device(x.device):
+    with _lib.on(x.device):
         _lib.call("tfb_router_prompt" if prompt and d % 32 == 0 else "tfb_router", x.data_ptr(), x.stride(0),
                   rows.data_ptr(), out.data_ptr(), m, d, ne, _stream(x))
     return out
@@ -73,7 +73,7 @@ def select_rows(logits: torch.Tensor, buf: MoEBuffers, top_k: int, experts: int)
         raise ValueError(f"{rows} rows of top-{top_k} do not fit buffers of {buf.rows} x {buf.slots}")
     if logits.dtype != torch.float32 or not logits.is_contiguous():
         raise ValueError("logits must be contiguous fp32")
-    with torch.cuda.device(logits.device):
+    with _lib.on(logits.device):
         _lib.call("tfb_select_rows", logits.data_ptr(), nl, buf.pick.data_ptr(), buf.wts.data_ptr(), rows, experts,
                   top_k, 1 if shared else 0, _stream(logits))
 
@@ -93,7 +93,7 @@ def select_sigmoid(logits: torch.Tensor, bias: torch.Tensor, pick: torch.Tensor,
     for t, dt in ((pick, torch.int32), (wts, torch.float32)):
         if t.dtype != dt or not t.is_contiguous() or t.shape[0] < rows or t.shape[1] != slots:
             raise ValueError(f"pick / wts must be contiguous [{rows}, {slots}] int32 / fp32")
-    with torch.cuda.device(logits.device):
+    with _lib.on(logits.device):
         _lib.call("tfb_select_sigmoid", logits.data_ptr(), nl, bias.data_ptr(), pick.data_ptr(), wts.data_ptr(), rows,
                   experts, top_k, shared_slots, float(scale), 1 if norm else 0, _stream(logits))
 
@@ -118,7 +118,7 @@ def select(logits: torch.Tensor, buf: MoEBuffers, top_k: int, experts: int,
         if buf.slots not in (top_k, top_k + 1) or rows > buf.rows or plan.slots != buf.slots:
             raise ValueError(f"{rows} rows of top-{top_k} do not fit buffers of {buf.rows} x {buf.slots}")
         plan.tile = tile if plan.prefill else plan.decode_tile
-        with torch.cuda.device(logits.device):
+        with _lib.on(logits.device):
             _lib.call("tfb_select_plan", logits.data_ptr(), nl, buf.pick.data_ptr(), buf.wts.data_ptr(), rows, experts,
                       top_k, 1 if shared else 0, plan.tile, plan.members.data_ptr(), plan.items.data_ptr(),
                       plan.counts.data_ptr(), _stream(logits))
@@ -159,7 +159,7 @@ def route(x: torch.Tensor, router_rows: torch.Tensor, buf: MoEBuffers, top_k: in
     if rows > route_rows(router_rows):
         raise ValueError(f"route: at most {route_rows(router_rows)} rows in one launch")
     plan.tile = tile if plan.prefill else plan.decode_tile
-    with torch.cuda.device(x.device):
+    with _lib.on(x.device):
         _lib.call("tfb_route", x.data_ptr(), x.stride(0), router_rows.data_ptr(), buf.logits.data_ptr(), rows, d, ne,
                   experts, top_k, 1 if shared else 0, buf.pick.data_ptr(), buf.wts.data_ptr(), plan.tile, 0,
                   plan.experts, plan.members.data_ptr(), plan.items.data_ptr(), plan.counts.data_ptr(),
@@ -215,7 +215,7 @@ def combine(y: torch.Tensor, wts: torch.Tensor, out: torch.Tensor | None = None)
         raise ValueError("combine: y must be contiguous fp32 or bf16, wts contiguous fp32")
     if out is None:
         out = torch.empty((rows, dims), dtype=torch.bfloat16, device=y.device)
-    with torch.cuda.device(y.device):
+    with _lib.on(y.device):
         _lib.call("tfb_combine", y.data_ptr(), 1 if y.dtype == torch.bfloat16 else 0, wts.data_ptr(), out.data_ptr(),
                   1 if out.dtype == torch.float32 else 0, rows, slots, dims, _stream(y))
     return out
@@ -237,7 +237,7 @@ def add_moe_norm(h: torch.Tensor, y: torch.Tensor, wt: torch.Tensor, w: torch.Te
         raise ValueError("add_moe_norm: wt must be contiguous fp32 [R, NS] with top_k <= NS")
     hn, out = torch.empty_like(h), torch.empty_like(h)
     xs = torch.empty((rows, d // 64), dtype=torch.float32, device=h.device)
-    with torch.cuda.device(h.device):
+    with _lib.on(h.device):
         _lib.call("tfb_add_moe_norm", h.data_ptr(), y.data_ptr(), 1 if y.dtype == torch.bfloat16 else 0, wt.data_ptr(),
                   w.contiguous().data_ptr(), hn.data_ptr(), out.data_ptr(), xs.data_ptr(), rows, d, slots, top_k,
                   float(eps), _stream(h))

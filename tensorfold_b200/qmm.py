@@ -86,9 +86,9 @@ def group_sums(x: torch.Tensor, gs: int = 64) -> torch.Tensor:
         raise ValueError("group_sums: x must be CUDA (M, K) bf16 with unit-stride rows")
     m, k = x.shape
     xs = torch.empty((m, k // gs), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on(x.device):
         _lib.call("tfb_group_sums", x.data_ptr(), x.stride(0), xs.data_ptr(), m, k, gs,
-                  torch.cuda.current_stream(x.device).cuda_stream)
+                  _lib.stream(x.device))
     return xs
 
 
@@ -160,11 +160,11 @@ def _slices(x: torch.Tensor, q: Q4, slices: int, part: torch.Tensor | None) -> t
     dst = part.reshape(-1)[:need].view(slices, m, q.n) if part is not None and not padded else \
         torch.empty((slices, m, q.n_pad), dtype=torch.float32, device=x.device)
     plan = _plan(m, x.device, False)
-    with torch.cuda.device(x.device):
+    with _lib.on(x.device):
         _lib.call("tfb_experts_run_slices", q.gs, x.data_ptr(), x.stride(0), 0, q.weight.data_ptr(), q.k // q.gs,
                   q.n_pad // grouped.COLS, plan.items.data_ptr(), plan.counts.data_ptr(), plan.members.data_ptr(),
                   dst.data_ptr(), q.n_pad, m, grouped.max_items(m, 1, plan.tile) * (q.n_pad // grouped.COLS),
-                  0 if q.scale_dtype == torch.bfloat16 else 1, plan.tile, torch.cuda.current_stream(x.device).cuda_stream)
+                  0 if q.scale_dtype == torch.bfloat16 else 1, plan.tile, _lib.stream(x.device))
     if not padded:
         return dst
     if part is None:
