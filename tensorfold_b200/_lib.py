@@ -86,6 +86,9 @@ def lib() -> ctypes.CDLL:
         fn = getattr(handle, name)
         fn.argtypes = args
         fn.restype = c_int
+    # A layer of few tokens is a chain of short kernels, and the gaps between plain launches are a good part of it: with
+    # programmatic launches one token through 128 experts takes 24 us instead of 27, thirteen tokens 62 instead of 74.
+    handle.tfb_set_pdl(1)
     return handle
 
 
@@ -129,6 +132,8 @@ def kernel_status(stream: int = 0) -> int:
 
 
 def set_pdl(on: bool) -> bool:
+    """Programmatic launches on (as the package starts) or off; returns the previous setting."""
+
     return bool(lib().tfb_set_pdl(1 if on else 0))
 
 
