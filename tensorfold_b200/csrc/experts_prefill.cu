@@ -18,8 +18,8 @@
 // gate/up moved 154 KB through it at 192 pairs (of it 64 KB A written and read) and the K loop ran at 0.91 us a stage;
 // without them and with two CTAs an SM (256 of the 512 tensor-memory columns each: 192 of accumulators, two A stages
 // of 32; under 113 KB of shared memory) one unit's start, epilogue and waits run under the other's K loop.
-// A B200 at 2048 tokens of 128 experts (2048 x 768, top 8): gate/up 220 -> 177 us, down 182 -> 116 us; at 317 tokens with
-// a shared expert 172 -> 124 and 143 -> 77 us.  What is left is instruction issue (two thirds of the slots, the ALU pipe
+// A B200 at 2048 tokens of 128 experts (2048 x 768, top 8): gate/up 220 -> 158 us, down 182 -> 110 us; at 317 tokens with
+// a shared expert 172 -> 119 and 143 -> 84 us.  What is left is instruction issue (two thirds of the slots, the ALU pipe
 // 60 % busy): about 1000 of the dequantising warps' instructions a stage against 256 cycles of MMA.
 // (Replaces src/tensorfold/cuda/experts_prefill.cu:31-195: prefill_kernel and its launch.)
 
@@ -259,9 +259,8 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
     const __nv_bfloat16* rowp[PF_GA_PER_THREAD];
 #pragma unroll
     for (int j = 0; j < PF_GA_PER_THREAD; ++j) {
-      const int r = r0 + 16 * j;
-      const int p = r < cnt ? out_row[r] : -1;
-      rowp[j] = p < 0 ? nullptr : X + (size_t)(slots ? p / slots : p) * x_stride + c * 8;
+      const int p = out_row[min(r0 + 16 * j, cnt - 1)];   // rows past the last repeat it: their columns are never stored
+      rowp[j] = X + (size_t)(slots ? p / slots : p) * x_stride + c * 8;
     }
     const uint32_t boff = (uint32_t)(r0 * 128 + ((c ^ (r0 & 7)) << 4));      // rows 16 apart share r & 7
     int s = 0, ph = 1, back = 0;                     // ph: a ring's first round finds every stage free
@@ -272,7 +271,8 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
 #pragma unroll
       for (int j = 0; j < PF_GA_PER_THREAD; ++j) {
         if (16 * j >= cnt) break;
-        if (rowp[j]) cp_async16(btile + j * (16 * 128), rowp[j] + g * GS);
+        cp_async16(btile + j * (16 * 128), rowp[j]);
+        rowp[j] += GS;
       }
       cp_async_commit();
       if (++s == sb) {
@@ -309,17 +309,12 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
       if (!ok) break;
       const uint8_t* blk = smem + SM::PACKED_OFFSET + sp * SM::PACKED_BYTES;
       uint2 w[4];
-      uint32_t sbw = 0u;
-      if (cbw < ncb) {
-        sbw = *reinterpret_cast<const uint32_t*>(blk + sb_at);
+      // (a block that the unit lacks: whatever the slot holds, its columns are never stored)
+      const uint32_t sbw = *reinterpret_cast<const uint32_t*>(blk + sb_at);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) w[u] = *reinterpret_cast<const uint2*>(blk + w_at + (((u + rot) & 3) << 4));
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) w[u] = make_uint2(0u, 0u);
-      }
+      for (int u = 0; u < 4; ++u) w[u] = *reinterpret_cast<const uint2*>(blk + w_at + (((u + rot) & 3) << 4));
       __syncwarp();
-      if (lane == 0) mbar_arrive(packed_free + sp);
+      mbar_arrive_if(packed_free + sp, lane == 0);
       uint2 v[4], x[4];                              // piece k = w[(k - rot) & 3]
 #pragma unroll
       for (int k = 0; k < 4; ++k) v[k] = (rot & 1) ? w[(k + 3) & 3] : w[k];
@@ -345,7 +340,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(a_ready + set);
+      mbar_arrive_if(a_ready + set, lane == 0);
     }
   }
   // ---------------- epilogue: the twelve dequantising and gathering warps ----------------
