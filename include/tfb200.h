@@ -234,6 +234,12 @@ int tfb_experts_prefill(int gs, int epi, const void* x, int64_t x_stride, int sl
                         const int32_t* items, const int32_t* counts, const int32_t* members, void* out, int n,
                         float limit, int64_t max_items, int sb_type, void* stream);
 
+/* The same over a plan whose items hold at most `tile` pairs (1..192): with 64 or fewer a build with three blocks an SM
+ * instead of two, for prompts with few pairs an expert.  A pair's bits do not depend on the tile. */
+int tfb_experts_prefill_tile(int gs, int epi, const void* x, int64_t x_stride, int slots, const void* w, int kg, int nb,
+                             const int32_t* items, const int32_t* counts, const int32_t* members, void* out, int n,
+                             float limit, int64_t max_items, int sb_type, int tile, void* stream);
+
 /* ---- EXL3 trellis-coded experts ------------------------------------------------------------------------------- */
 /* Trellises are int16 [K/16, N/16, 8 * k2] (k2 = half-bits a value, 2..16), read in place; cb 0 = 3inst, 1 = mcg,
  * 2 = mul1; suh / svh are fp16 [E, n].  K and N are multiples of 128. */

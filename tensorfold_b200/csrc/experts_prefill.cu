@@ -17,9 +17,10 @@
 // What bounds it: shared-memory bandwidth and tensor issue, about even.  With the A tiles in shared memory a stage of
 // gate/up moved 154 KB through it at 192 pairs (of it 64 KB A written and read) and the K loop ran at 0.91 us a stage;
 // without them and with two CTAs an SM (256 of the 512 tensor-memory columns each: 192 of accumulators, two A stages
-// of 32; under 113 KB of shared memory) one unit's start, epilogue and waits run under the other's K loop.
+// of 32; under 113 KB of shared memory; three CTAs in the build for items of up to 64 pairs) one unit's start, epilogue
+// and waits run under the others' K loops.
 // A B200 at 2048 tokens of 128 experts (2048 x 768, top 8): gate/up 220 -> 158 us, down 182 -> 110 us; at 317 tokens with
-// a shared expert 172 -> 119 and 143 -> 84 us.  What is left is instruction issue (two thirds of the slots, the ALU pipe
+// a shared expert (20 pairs an expert, items of 64) 172 -> 93 and 143 -> 65 us.  What is left is instruction issue (two thirds of the slots, the ALU pipe
 // 60 % busy): about 1000 of the dequantising warps' instructions a stage against 256 cycles of MMA.
 // (Replaces src/tensorfold/cuda/experts_prefill.cu:31-195: prefill_kernel and its launch.)
 
@@ -30,32 +31,44 @@ namespace tfb {
 
 constexpr int PF_ROWS = 128;            // weight rows a unit (MMA M)
 constexpr int PF_MAXP = 192;            // pairs an item may hold (MMA N)
+constexpr int PF_SMALL_MAXP = 64;       // the same in the build for plans of small items
 constexpr int PF_DQ_WARPS = 8;          // warps 0-7: dequantise (two sets of four), then the epilogue
-constexpr int PF_GA_WARPS = 4;          // warps 8-11: gather the pairs' input rows
-constexpr int PF_MMA_WARP = 12, PF_COPY_WARP = 13;
-constexpr int PF_THREADS = 14 * 32;
-constexpr int PF_GA_PER_THREAD = PF_MAXP * 8 / (PF_GA_WARPS * 32);   // 16-byte chunks a gather thread a stage
-constexpr int PF_TMEM_COLS = 256;       // a CTA's share of the tensor memory
-constexpr int PF_A_COL = PF_MAXP;       // its A stages: 2 x 32 columns behind the accumulators
+
+// What the two builds differ in.  Items of up to 192 pairs: two CTAs an SM.  Items of up to 64: half the accumulators and a
+// third of the B ring, two gathering warps - three CTAs, because a unit of few pairs is mostly start, latency and epilogue.
+// (317 tokens, top 8 of 128 and a shared expert: gate/up 119 us in the large build, 93 in this one, down 84 and 65.)
+template <int MAXP>
+struct PrefillShape {
+  static constexpr int CTAS = MAXP > PF_SMALL_MAXP ? 2 : 3;                    // an SM
+  static constexpr int GA_WARPS = MAXP > PF_SMALL_MAXP ? 4 : 2;               // warps 8 ..: gather the pairs' input rows
+  static constexpr int MMA_WARP = PF_DQ_WARPS + GA_WARPS, COPY_WARP = MMA_WARP + 1;
+  static constexpr int THREADS = (COPY_WARP + 1) * 32;
+  static constexpr int GA_ROWS = GA_WARPS * 4;                                 // rows a pass of the gathering warps
+  static constexpr int EPI_PARTS = MAXP > PF_SMALL_MAXP ? 3 : 2;              // warps a lane quarter in the epilogue
+  static constexpr int A_COL = MAXP;                                           // tensor memory: accumulators, two A stages
+  static constexpr int TMEM_COLS = MAXP + 64;
+};
 
 template <int M>
 constexpr int PF_CB = PF_ROWS / COLS / M;   // packed column blocks a unit
 
 // Two rings in shared memory: the B tiles (whole tiles of the item's own height, so items of fewer pairs get more
 // stages) and the packed blocks as they come from HBM.
+template <int MAXP>
 struct PrefillSmem {
   static constexpr int SP = 8;
-  static constexpr int B_BYTES = 3 * PF_MAXP * 128;
+  static constexpr int B_BYTES = 3 * MAXP * 128;
   static constexpr int SB_MAX = 6;
   static constexpr int PACKED_BYTES = PF_ROWS / COLS * BLOCK_BYTES;
   static constexpr int PACKED_OFFSET = B_BYTES;
-  static constexpr int TABLE_OFFSET = PACKED_OFFSET + SP * PACKED_BYTES;   // int out_row[PF_MAXP]
-  static constexpr int BAR_OFFSET = (TABLE_OFFSET + PF_MAXP * 4 + 15) / 16 * 16;
+  static constexpr int TABLE_OFFSET = PACKED_OFFSET + SP * PACKED_BYTES;   // int out_row[MAXP]
+  static constexpr int BAR_OFFSET = (TABLE_OFFSET + MAXP * 4 + 15) / 16 * 16;
   static constexpr int NBARS = 2 * SP + 2 * 2 + 2 * SB_MAX + 1;
   static constexpr int TMEM_OFFSET = BAR_OFFSET + NBARS * 8;
   static constexpr int TOTAL = TMEM_OFFSET + 16 + 1024;         // + slack to align the tiles to 1024 bytes
+  static_assert(PrefillShape<MAXP>::CTAS * (TOTAL + 1024) <= 228 * 1024, "the CTAs share an SM's shared memory");
+  static_assert(PrefillShape<MAXP>::CTAS * PrefillShape<MAXP>::TMEM_COLS <= 512, "and its tensor memory");
 };
-static_assert(2 * (PrefillSmem::TOTAL + 1024) <= 228 * 1024, "two CTAs share an SM");
 
 // ---- tcgen05 wrappers ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
@@ -147,12 +160,13 @@ __device__ __forceinline__ uint32_t prefill_pair(uint32_t v, uint32_t sb) {
   }
 }
 
-template <int M, int EPI, int SB>
-__global__ void __launch_bounds__(PF_THREADS, 2)
+template <int M, int EPI, int SB, int MAXP>
+__global__ void __launch_bounds__(PrefillShape<MAXP>::THREADS, PrefillShape<MAXP>::CTAS)
 prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots, const uint8_t* __restrict__ W, int KG,
                int NB, const int* __restrict__ items, const int* __restrict__ counts, const int* __restrict__ members,
                void* __restrict__ out, int N, float limit) {
-  using SM = PrefillSmem;
+  using SM = PrefillSmem<MAXP>;
+  using SH = PrefillShape<MAXP>;
   constexpr int SP = SM::SP, CB = PF_CB<M>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -181,7 +195,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
       mbar_init(a_free + s, 1);
     }
     for (int s = 0; s < SM::SB_MAX; ++s) {
-      mbar_init(b_ready + s, PF_GA_WARPS * 32);
+      mbar_init(b_ready + s, SH::GA_WARPS * 32);
       mbar_init(b_free + s, 1);
     }
     mbar_init(acc_ready, 1);
@@ -191,13 +205,13 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
   pdl_wait();
   after_wait(X, items, counts, members);
   const bool live = it < ld_dep(counts);          // uniform over the CTA
-  if (live && warp == PF_MMA_WARP) tmem_alloc(tmem_slot, PF_TMEM_COLS);
+  if (live && warp == SH::MMA_WARP) tmem_alloc(tmem_slot, SH::TMEM_COLS);
   int e = 0, first = 0, cnt = 0;
   if (live) {
     e = ld_dep(items + 3 * it);
     first = ld_dep(items + 3 * it + 1);
-    cnt = min(ld_dep(items + 3 * it + 2), PF_MAXP);
-    for (int i = tid; i < PF_MAXP; i += PF_THREADS) out_row[i] = i < cnt ? ld_dep(members + first + i) : -1;
+    cnt = min(ld_dep(items + 3 * it + 2), MAXP);
+    for (int i = tid; i < MAXP; i += SH::THREADS) out_row[i] = i < cnt ? ld_dep(members + first + i) : -1;
   }
   tc_fence_before();
   __syncthreads();
@@ -210,7 +224,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
   const int cb0 = ct * CB, ncb = min(CB, NB - cb0);              // packed column blocks of this unit
   bool ok = true;
 
-  if (warp == PF_COPY_WARP) {
+  if (warp == SH::COPY_WARP) {
     // ---------------- packed weights: HBM -> the packed ring, a lane a column block, as far ahead as the ring allows
     const size_t cb_stride = (size_t)KG * (M * BLOCK_BYTES);
     const uint8_t* wsrc = W + (size_t)e * NB * cb_stride + (size_t)(cb0 + lane) * cb_stride;
@@ -228,7 +242,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
     if (!ok && lane == 0)                            // give the copies in flight a while to land
       for (int f = max(0, g - SP); f < g; ++f) mbar_wait_for(packed_full + f % SP, (f / SP) & 1, 10000000ull);
     __syncwarp();
-  } else if (warp == PF_MMA_WARP) {
+  } else if (warp == SH::MMA_WARP) {
     // ---------------- MMA issue: one lane ----------------
     if (lane == 0) {
       const uint32_t idesc = umma_idesc(nmma);
@@ -239,7 +253,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
         if (!ok) break;
         tc_fence_after();
         const uint64_t desc = desc0 + (uint32_t)(s * (b_bytes >> 4));
-        const uint32_t a = tmem_base + PF_A_COL + (g & 1) * 32;
+        const uint32_t a = tmem_base + SH::A_COL + (g & 1) * 32;
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) umma_ta(tmem_base, a + ks * 8, desc + 2 * ks, idesc, (g | ks) ? 1u : 0u);
         umma_commit(a_free + (g & 1));
@@ -254,24 +268,25 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
     __syncwarp();
   } else if (warp >= PF_DQ_WARPS) {
     // ---------------- warps 8-11: gather the pairs' input rows into the swizzled B tiles ----------------
-    // thread -> chunk c of rows r0, r0 + 16, ...: the row pointers stay in registers for the whole K loop
+    // thread -> chunk c of rows r0, r0 + GA_ROWS, ...: the row pointers stay in registers for the whole K loop
+    constexpr int GA_PER = MAXP / SH::GA_ROWS;       // 16-byte chunks a thread a stage
     const int gt = tid - PF_DQ_WARPS * 32, c = gt & 7, r0 = gt >> 3;
-    const __nv_bfloat16* rowp[PF_GA_PER_THREAD];
+    const __nv_bfloat16* rowp[GA_PER];
 #pragma unroll
-    for (int j = 0; j < PF_GA_PER_THREAD; ++j) {
-      const int p = out_row[min(r0 + 16 * j, cnt - 1)];   // rows past the last repeat it: their columns are never stored
+    for (int j = 0; j < GA_PER; ++j) {
+      const int p = out_row[min(r0 + SH::GA_ROWS * j, cnt - 1)];   // rows past the last repeat it: their columns are never stored
       rowp[j] = X + (size_t)(slots ? p / slots : p) * x_stride + c * 8;
     }
-    const uint32_t boff = (uint32_t)(r0 * 128 + ((c ^ (r0 & 7)) << 4));      // rows 16 apart share r & 7
+    const uint32_t boff = (uint32_t)(r0 * 128 + ((c ^ (r0 & 7)) << 4));      // rows GA_ROWS apart share r & 7
     int s = 0, ph = 1, back = 0;                     // ph: a ring's first round finds every stage free
     for (int g = 0; g < KG && ok; ++g) {
       if (g >= sb) ok = mbar_wait_warp(b_free + s, ph);
       if (!ok) break;
       uint8_t* btile = smem + s * b_bytes + boff;
 #pragma unroll
-      for (int j = 0; j < PF_GA_PER_THREAD; ++j) {
-        if (16 * j >= cnt) break;
-        cp_async16(btile + j * (16 * 128), rowp[j]);
+      for (int j = 0; j < GA_PER; ++j) {
+        if (SH::GA_ROWS * j >= cnt) break;
+        cp_async16(btile + j * (SH::GA_ROWS * 128), rowp[j]);
         rowp[j] += GS;
       }
       cp_async_commit();
@@ -302,7 +317,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
     const int rot = (t >> 1) * 2 + ((gq >> 1) & 1);
     const int at = cbw * (M * BLOCK_BYTES) + mm * BLOCK_BYTES;
     const int w_at = at + tt * TILE_BYTES + gq * 64 + hi * 8, sb_at = at + SB_OFFSET + gq * 16 + (2 * tt + hi) * 4;
-    const uint32_t a_dst = tmem_base + ((uint32_t)(q * 32) << 16) + PF_A_COL + set * 32;
+    const uint32_t a_dst = tmem_base + ((uint32_t)(q * 32) << 16) + SH::A_COL + set * 32;
     for (int g = set; g < KG && ok; g += 2) {
       const int sp = g % SP;
       ok = mbar_wait_warp(packed_full + sp, (g / SP) & 1);
@@ -343,11 +358,11 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
       mbar_arrive_if(a_ready + set, lane == 0);
     }
   }
-  // ---------------- epilogue: the twelve dequantising and gathering warps ----------------
-  // TMEM lane quarter warp & 3, a weight row a lane (numbered as the dequantising warps do); the three warps of a
-  // quarter take a third of the pairs each, 16 pairs a load.  Gate and up rows of a column sit in lanes 2 apart: of
+  // ---------------- epilogue: the dequantising warps, and the four gathering warps of the large build ----------------
+  // TMEM lane quarter warp & 3, a weight row a lane (numbered as the dequantising warps do); the two or three warps
+  // of a quarter take a part of the pairs each, 16 pairs a load.  Gate and up rows of a column sit in lanes 2 apart: of
   // two neighbouring pairs the gate lane forms the first and the up lane the second, one exchange for both.
-  if (warp < PF_DQ_WARPS + PF_GA_WARPS) {
+  if (warp < 4 * SH::EPI_PARTS) {
     if (ok) ok = mbar_wait_warp(acc_ready, 0);
     if (ok) {
       tc_fence_after();
@@ -355,7 +370,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
       const int col = M == 1 ? ct * PF_ROWS + q * 32 + (t >> 1) * 16 + (t & 1) * 8 + gq
                              : ct * (PF_ROWS / 2) + q * 16 + (t & 1) * 8 + gq;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
-      const int blocks = nmma / 16, per = (blocks + 2) / 3;
+      const int blocks = nmma / 16, per = (blocks + SH::EPI_PARTS - 1) / SH::EPI_PARTS;
       const int jb = min(blocks, part * per) * 16, je = min(blocks, (part + 1) * per) * 16;
       for (int j0 = jb; j0 < je; j0 += 16) {
         uint32_t a[16];
@@ -408,15 +423,15 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
   pdl_launch_dependents();
   tc_fence_before();
   __syncthreads();
-  if (warp == PF_MMA_WARP) tmem_dealloc(tmem_base, PF_TMEM_COLS);
+  if (warp == SH::MMA_WARP) tmem_dealloc(tmem_base, SH::TMEM_COLS);
 }
 
-template <int M, int EPI, int SB>
+template <int M, int EPI, int SB, int MAXP>
 int launch_prefill(const void* x, int64_t x_stride, int slots, const void* w, int kg, int nb, const int* items,
                    const int* counts, const int* members, void* out, int n, float limit, int64_t max_items,
                    cudaStream_t stream) {
-  using SM = PrefillSmem;
-  auto* kern = prefill_kernel<M, EPI, SB>;
+  using SM = PrefillSmem<MAXP>;
+  auto* kern = prefill_kernel<M, EPI, SB, MAXP>;
   static bool configured[64] = {false};
   int dev = 0;
   TFB_CUDA(cudaGetDevice(&dev), "experts_prefill: cudaGetDevice");
@@ -428,7 +443,7 @@ int launch_prefill(const void* x, int64_t x_stride, int slots, const void* w, in
   }
   const int64_t grid = max_items * ((nb + PF_CB<M> - 1) / PF_CB<M>);
   if (grid >= (int64_t(1) << 31)) return fail(TFB_ERR_ARG, "experts_prefill: too many units");
-  return check_cuda(launch(kern, dim3((unsigned)grid), dim3(PF_THREADS), (size_t)SM::TOTAL, stream,
+  return check_cuda(launch(kern, dim3((unsigned)grid), dim3(PrefillShape<MAXP>::THREADS), (size_t)SM::TOTAL, stream,
                            static_cast<const __nv_bfloat16*>(x), x_stride, slots, static_cast<const uint8_t*>(w), kg,
                            nb, items, counts, members, out, n, limit),
                     "experts_prefill");
@@ -438,11 +453,9 @@ int launch_prefill(const void* x, int64_t x_stride, int slots, const void* w, in
 
 using namespace tfb;
 
-// Grouped 4-bit expert matmul, prefill form, over a plan whose items hold at most 192 pairs.  Arguments as the
-// reference extension's `prefill` (src/tensorfold/cuda/experts.cpp:50-56); max_items = an upper bound of the items.
-extern "C" int tfb_experts_prefill(int gs, int epi, const void* x, int64_t x_stride, int slots, const void* w, int kg,
-                                   int nb, const int32_t* items, const int32_t* counts, const int32_t* members,
-                                   void* out, int n, float limit, int64_t max_items, int sb_type, void* stream) {
+static int experts_prefill(int gs, int epi, const void* x, int64_t x_stride, int slots, const void* w, int kg, int nb,
+                           const int32_t* items, const int32_t* counts, const int32_t* members, void* out, int n,
+                           float limit, int64_t max_items, int sb_type, int tile, void* stream) {
   TFB_REQUIRE(gs == GS, "experts_prefill: groups of %d inputs only, not %d", GS, gs);
   TFB_REQUIRE(x && w && items && counts && members && out, "experts_prefill: null pointer");
   TFB_REQUIRE(kg >= 1 && nb >= 1 && n == nb * COLS, "experts_prefill: n must be the column blocks times %d", COLS);
@@ -452,16 +465,41 @@ extern "C" int tfb_experts_prefill(int gs, int epi, const void* x, int64_t x_str
   TFB_REQUIRE(slots >= 0 && max_items >= 0, "experts_prefill: bad slots or item count");
   TFB_REQUIRE(sb_type == SB_BF16 || sb_type == SB_FP16, "experts_prefill: scales are bf16 (0) or fp16 (1), not %d",
               sb_type);
+  TFB_REQUIRE(tile >= 1 && tile <= PF_MAXP, "experts_prefill: items of 1..%d pairs, not %d", PF_MAXP, tile);
   if (max_items == 0) return TFB_OK;
   auto st = static_cast<cudaStream_t>(stream);
-#define TFB_PRE(EPI_, M_)                                                                                           \
-  if (epi == EPI_)                                                                                                  \
-    return sb_type == SB_BF16                                                                                       \
-               ? launch_prefill<M_, EPI_, SB_BF16>(x, x_stride, slots, w, kg, nb, items, counts, members, out, n,   \
-                                                   limit, max_items, st)                                            \
-               : launch_prefill<M_, EPI_, SB_FP16>(x, x_stride, slots, w, kg, nb, items, counts, members, out, n,   \
-                                                   limit, max_items, st);
+#define TFB_PRE2(EPI_, M_, SB_)                                                                                        \
+  return tile <= PF_SMALL_MAXP                                                                                         \
+             ? launch_prefill<M_, EPI_, SB_, PF_SMALL_MAXP>(x, x_stride, slots, w, kg, nb, items, counts, members, out, \
+                                                            n, limit, max_items, st)                                   \
+             : launch_prefill<M_, EPI_, SB_, PF_MAXP>(x, x_stride, slots, w, kg, nb, items, counts, members, out, n,    \
+                                                      limit, max_items, st)
+#define TFB_PRE(EPI_, M_)                              \
+  if (epi == EPI_) {                                   \
+    if (sb_type == SB_BF16) TFB_PRE2(EPI_, M_, SB_BF16); \
+    TFB_PRE2(EPI_, M_, SB_FP16);                       \
+  }
   TFB_PRE(EPI_F32, 1) TFB_PRE(EPI_RELU2, 1) TFB_PRE(EPI_SWIGLU, 2) TFB_PRE(EPI_BF16, 1)
 #undef TFB_PRE
+#undef TFB_PRE2
   return fail(TFB_ERR_ARG, "experts_prefill: no kernel for epilogue %d", epi);
+}
+
+// Grouped 4-bit expert matmul, prefill form, over a plan whose items hold at most 192 pairs.  Arguments as the
+// reference extension's `prefill` (src/tensorfold/cuda/experts.cpp:50-56); max_items = an upper bound of the items.
+extern "C" int tfb_experts_prefill(int gs, int epi, const void* x, int64_t x_stride, int slots, const void* w, int kg,
+                                   int nb, const int32_t* items, const int32_t* counts, const int32_t* members,
+                                   void* out, int n, float limit, int64_t max_items, int sb_type, void* stream) {
+  return experts_prefill(gs, epi, x, x_stride, slots, w, kg, nb, items, counts, members, out, n, limit, max_items, sb_type,
+                         PF_MAXP, stream);
+}
+
+// The same over a plan whose items hold at most `tile` pairs (1..192): with 64 or fewer a build with less of an SM to a
+// CTA, three of them an SM.  A pair's bits do not depend on the tile.
+extern "C" int tfb_experts_prefill_tile(int gs, int epi, const void* x, int64_t x_stride, int slots, const void* w, int kg,
+                                        int nb, const int32_t* items, const int32_t* counts, const int32_t* members,
+                                        void* out, int n, float limit, int64_t max_items, int sb_type, int tile,
+                                        void* stream) {
+  return experts_prefill(gs, epi, x, x_stride, slots, w, kg, nb, items, counts, members, out, n, limit, max_items, sb_type,
+                         tile, stream);
 }

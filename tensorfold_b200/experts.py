@@ -19,6 +19,8 @@ COLS = 8 * NTW           # output columns a block
 TILE = 8                 # pairs an item holds (decode form): one mma tile of pairs
 WIDE_TILE = 16           # the decode form's other item size: two mma tiles share one dequantisation
 PREFILL_TILE = 192       # pairs a prompt item holds: the tensor-core tile's N
+SMALL_PREFILL_TILE = 64  # the same for the prompt kernel's build with three blocks an SM
+SMALL_PREFILL_FROM = 32  # pairs an expert on average up to which a prompt sorts into the small items
 SMALL = 1024             # kept for callers that size scratch by it; this library's plan is one launch at any size
 BLOCK = 288              # int32 words a block of 64 inputs x 32 columns: 1024 B of nibbles + 128 B of scale/bias
 
@@ -137,6 +139,15 @@ def max_items(pairs: int, experts: int, tile: int = TILE) -> int:
 
     used = min(pairs, experts)
     return used + (pairs - used) // tile
+
+
+def prompt_tile(pairs: int, experts: int) -> int:
+    """Pairs an item of a prompt's plan holds.  With few pairs an expert a unit of the prompt kernel is mostly start, latency
+    and epilogue, and three smaller blocks an SM hide more of it than two; with many, larger items dequantise an expert's
+    weights fewer times.  At 20 pairs an expert (and one shared expert of 317) a layer takes 175 us with the small items, 220
+    with the large.  A pair's bits depend on neither."""
+
+    return SMALL_PREFILL_TILE if pairs <= SMALL_PREFILL_FROM * experts else PREFILL_TILE
 
 
 class Plan:
@@ -260,9 +271,9 @@ def _run(epi: int, x: torch.Tensor, slots: int, w: torch.Tensor, kg: int, nb: in
         raise ValueError("w must be contiguous")
     with _lib.on(x.device):
         if prefill:
-            _lib.call("tfb_experts_prefill", ex.gs, epi, x.data_ptr(), x.stride(0), slots, w.data_ptr(), kg, nb,
+            _lib.call("tfb_experts_prefill_tile", ex.gs, epi, x.data_ptr(), x.stride(0), slots, w.data_ptr(), kg, nb,
                       plan.items.data_ptr(), plan.counts.data_ptr(), plan.members.data_ptr(), out.data_ptr(), n,
-                      float(limit), items, _SB[ex.scale_dtype], _stream(x))
+                      float(limit), items, _SB[ex.scale_dtype], plan.tile, _stream(x))
         else:
             _lib.call("tfb_experts_run_tile", ex.gs, epi, x.data_ptr(), x.stride(0), slots, w.data_ptr(), kg, nb,
                       plan.items.data_ptr(), plan.counts.data_ptr(), plan.members.data_ptr(), out.data_ptr(), n,

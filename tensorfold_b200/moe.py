@@ -175,7 +175,7 @@ def _route_any(x: torch.Tensor, router_rows: torch.Tensor, buf: MoEBuffers, top_
         route(x, router_rows, buf, top_k, experts)
         return 1
     router(x, router_rows, buf.logits[:rows], prompt=buf.plan.prefill)
-    select(buf.logits[:rows], buf, top_k, experts)
+    select(buf.logits[:rows], buf, top_k, experts, grouped.prompt_tile(rows * buf.slots, buf.plan.experts))
     return 2 if rows <= fused_select_rows() else 3
 
 

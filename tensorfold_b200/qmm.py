@@ -99,7 +99,8 @@ def _plan(m: int, device: torch.device, prefill: bool) -> grouped.Plan:
     plan = _PLANS.get(key)
     if plan is None:
         plan = grouped.Plan(m, 1, 1, device, prefill=prefill, decode_tile=bucket(m))
-        grouped.route(torch.zeros((m, 1), dtype=torch.int32, device=device), plan, grouped.PREFILL_TILE)
+        grouped.route(torch.zeros((m, 1), dtype=torch.int32, device=device), plan,
+                      grouped.prompt_tile(m, 1))
         torch.cuda.current_stream(device).synchronize()
         _PLANS[key] = plan
     return plan
