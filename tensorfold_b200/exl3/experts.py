@@ -26,7 +26,12 @@ K2_SUPPORTED = tuple(range(2, 17))   # half-bits a value: 1..8 bits and every ha
 LAUNCHES_PER_CALL = 4             # kernels one ``routed`` call with weights enqueues (3 without)
 ITEM_PAIRS = 16                   # pairs an item of the sort holds: two mma tiles share one decoded weight tile
 WIDE_ITEM_PAIRS = 32              # the same for the kernel's tensor-memory form, for calls with many pairs an expert
-WIDE_FROM = 12                    # pairs an expert on average from which a call sorts into the wide items
+# Pairs an expert on average from which a call sorts into the wide items (either way the same bits; whole calls measured,
+# narrow against wide items): widths 5 bits 12 pairs 292 / 292 us, 14 pairs 322 / 300; 3 bits 12 pairs 157 / 164, 16 pairs
+# 195 / 171.  At 4.00 bits the narrow items have a kernel build of their own: 14 pairs 274 / 303.  Where the widths differ
+# the narrow items run the build with short loops: 4.8 pairs 992 / 1002, 6.4 pairs 1023 / 1013, 11 pairs 1181 / 1061 - in a
+# launch of several waves (below that: not measured, the one-width line).
+WIDE_FROM, WIDE_FROM_FOUR, WIDE_FROM_MIXED = 14, 16, 6
 
 # (16-column tiles a block, K-slice warps, K splits across blocks, tiles in flight): this library's one setting.
 # The split is by shape only; partial sums meet in warp order inside the block, so there is one split.
@@ -158,13 +163,22 @@ def default_config(K: int, N: int, gateup: bool) -> tuple[int, int, int, int]:
     return CONFIG
 
 
-def item_pairs(pairs: int, experts: int) -> int:
+def item_pairs(pairs: int, experts: int, wide_from: float = WIDE_FROM) -> int:
     """Pairs an item of a call's sort holds: a function of the call's shape alone (a pair's bits depend on neither)."""
 
-    return WIDE_ITEM_PAIRS if pairs >= WIDE_FROM * experts else ITEM_PAIRS
+    return WIDE_ITEM_PAIRS if pairs >= wide_from * experts else ITEM_PAIRS
+
+
+def wide_from(ex: "Exl3RoutedExperts", pairs: int) -> float:
+    """The line for ``item_pairs`` of a layer."""
+
+    if ex.mixed and min(pairs, ex.count) * (ex.width // 128) * 2 >= WIDE_WAVES_BLOCKS:
+        return WIDE_FROM_MIXED
+    return WIDE_FROM_FOUR if ex.k2_gu == ex.k2_d == (8, 8) else WIDE_FROM
 
 
 COMPACT_MIXED = True              # projections of mixed widths run the trellis kernel's build with short loops (same bits)
+WIDE_WAVES_BLOCKS = 1184          # blocks of the wide items' kernel that fill a B200 four times (148 SMs x 2)
 CROWDED_BLOCKS = 592              # thread blocks from which an SM of a B200 holds four of a launch at once
 FILL_BLOCKS = 1480                # thread blocks that fill a B200 twice over (148 SMs x 5 blocks x 2)
 
@@ -262,7 +276,8 @@ def routed(x: torch.Tensor, pick: torch.Tensor, wts: torch.Tensor | None, ex: Ex
         raise ValueError("act_mode is ACT_BF16 or ACT_F32")
     st, items = _stream(x), max_items(pairs, ex.count)
     # `group` sorts into the narrow items; an expert-parallel rank expects only its share of the pairs
-    per_item = item_pairs(int(pairs * share), ex.count) if group_first else ITEM_PAIRS
+    expected = int(pairs * share)
+    per_item = item_pairs(expected, ex.count, wide_from(ex, expected)) if group_first else ITEM_PAIRS
     sort = (s.sort_members.data_ptr(), s.sort_items.data_ptr(), s.sort_counts.data_ptr())
     # the one width of a projection's tensors; or -1: they differ and the launch is large enough for blocks of several
     # widths to share an SM (the kernels then run a build with short loops); or 0: they differ, a small launch
