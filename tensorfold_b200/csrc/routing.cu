@@ -326,7 +326,7 @@ select_sigmoid_kernel(const float* __restrict__ L, int NL, const float* __restri
   const int r = blockIdx.x * S_WARPS + (threadIdx.x >> 5);
   if (r >= T) return;
   pdl_wait();
-  after_wait(L);
+  after_wait(L, bias);
   const int slots = top_k + shared;
   const float* Lr = L + (size_t)r * NL;
   uint32_t key[VPL];
@@ -724,7 +724,7 @@ combine_kernel(const TY* __restrict__ y, const float* __restrict__ wts, TO* __re
   const int d = (blockIdx.y * 256 + threadIdx.x) * 4;
   if (d >= D) return;
   pdl_wait();
-  after_wait(y, wts);
+  after_wait(y, wts, pick);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (int s = 0; s < S; ++s) {
     if (pick != nullptr) {
@@ -773,7 +773,7 @@ add_moe_norm_kernel(const __nv_bfloat16* __restrict__ h, const TY* __restrict__ 
   __shared__ float warp_sq[AMN_THREADS / 32];
   const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
   pdl_wait();
-  after_wait(h, y, wt);
+  after_wait(h, y, wt, w);
   float hv[AMN_MAX_PER_THREAD][4];
   float sq = 0.f;
 #pragma unroll
