@@ -1094,7 +1094,7 @@ exl3_rot_out_kernel(const float* __restrict__ z, const __half* __restrict__ svh,
   const int64_t units = (int64_t)M * nblk;
   const int64_t warps = (int64_t)gridDim.x * 8;
   pdl_wait();
-  after_wait(z);
+  after_wait(z, svh, bias);
   for (int64_t u0 = 4 * ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)); u0 < units; u0 += 4 * warps) {
     const bool have = u0 + quad < units;              // the transform's shuffles need every lane: an idle one repeats u0
     const int64_t u = have ? u0 + quad : u0;

@@ -3,7 +3,8 @@
 ``griddepcontrol.wait`` alone does not hold the compiler to that: a load through a ``const __restrict__`` parameter counts
 as invariant and may be moved above it.  ``after_wait`` names the pointers that are re-materialised behind the wait; this
 reads the sources and asks that no such parameter of a waiting kernel is missing from it.  Exempt are parameters that are
-read by volatile asm alone (``ldg_nc``, bulk copies), which keeps its place behind the wait."""
+read by volatile asm alone (``ldg_nc``, bulk copies), which keeps its place behind the wait, and those whose addresses
+are computed from values that were read behind it."""
 
 import re
 from pathlib import Path
@@ -11,8 +12,10 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "tensorfold_b200" / "csrc"
-FILES = ["routing.cu"]
+FILES = ["exl3.cu", "routing.cu"]
 VOLATILE_READS = {"router_kernel": {"W"}, "router_rows_kernel": {"W"}, "router_mma_kernel": {"W"}, "route_kernel": {"W"}}
+# addresses that hang on a value read behind the wait: the input scales of the pair's expert
+DEPENDENT_ADDRESSES = {"exl3_prologue_kernel": {"suh0", "suh1"}}
 
 
 def kernels(text: str) -> list[tuple[str, str, str]]:
@@ -40,7 +43,7 @@ def untied(name: str, params: str, body: str) -> set[str]:
         return set()
     invariant = {p.split()[-1].lstrip("*&") for p in params.split(",") if "__restrict__" in p and "const" in p}
     tied = {n.strip() for call in re.findall(r"after_wait\(([^)]*)\)", body) for n in call.split(",")}
-    return invariant - tied - VOLATILE_READS.get(name, set())
+    return invariant - tied - VOLATILE_READS.get(name, set()) - DEPENDENT_ADDRESSES.get(name, set())
 
 
 @pytest.mark.parametrize("file", FILES)
