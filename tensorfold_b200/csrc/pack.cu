@@ -102,6 +102,7 @@ dequant_kernel(const uint32_t* __restrict__ blocks, void* __restrict__ out, int 
 __global__ void __launch_bounds__(128)
 group_sums_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, float* __restrict__ xs, int M, int KG) {
   pdl_wait();
+  after_wait(x);
   const int lane = threadIdx.x & 31;
   const int64_t unit = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (unit < (int64_t)M * KG) {

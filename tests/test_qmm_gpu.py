@@ -125,3 +125,21 @@ def test_k_slices_apart_add_up_to_the_reduced_bits(n, k, m):
     part = torch.full((sk * m * n + 7,), 3.0, device=DEV)
     again = qmm.matmul(x, q, reduce=False, part=part)
     assert again.data_ptr() == part.data_ptr() and torch.equal(again, got) and bool((part[sk * m * n:] == 3.0).all())
+
+
+def test_group_sums_follow_the_kernel_before_them(pdl):
+    """Right behind the kernel that writes their rows, with other rows each time: the sums of these rows, not of the ones
+    the buffer held before.  Exact: rows of small whole numbers."""
+
+    from tensorfold_b200 import moe, qmm
+
+    m, k = 96, 4096
+    out, wts = torch.zeros((m, k), dtype=torch.bfloat16, device=DEV), torch.ones((m, 1), device=DEV)
+    ys = [torch.randint(-8, 9, (m, 1, k), generator=torch.Generator(device=DEV).manual_seed(i), device=DEV).float()
+          for i in range(8)]
+    got = []
+    for y in ys:
+        moe.combine(y, wts, out)
+        got.append(qmm.group_sums(out))
+    for y, xs in zip(ys, got):
+        assert torch.equal(xs, y.view(m, k // 64, 64).sum(-1))

@@ -12,7 +12,7 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "tensorfold_b200" / "csrc"
-FILES = ["exl3.cu", "routing.cu"]
+FILES = ["exl3.cu", "pack.cu", "routing.cu"]
 VOLATILE_READS = {"router_kernel": {"W"}, "router_rows_kernel": {"W"}, "router_mma_kernel": {"W"}, "route_kernel": {"W"}}
 # addresses that hang on a value read behind the wait: the input scales of the pair's expert
 DEPENDENT_ADDRESSES = {"exl3_prologue_kernel": {"suh0", "suh1"}}
