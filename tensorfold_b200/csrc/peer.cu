@@ -88,6 +88,7 @@ __device__ __forceinline__ bool step_failed() { return *reinterpret_cast<volatil
 __global__ void __launch_bounds__(256)
 peer_stage_kernel(const uint4* __restrict__ x_local, uint8_t* __restrict__ window, int64_t x_offset, int64_t x_bytes) {
   pdl_wait();
+  after_wait(x_local);
   uint4* dst = reinterpret_cast<uint4*>(window + x_offset);
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < x_bytes / 16; i += (int64_t)gridDim.x * 256) dst[i] = x_local[i];
   pdl_launch_dependents();
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(256)
 peer_gather_kernel(uint8_t* const* __restrict__ windows, int rank, int world, PeerSegs segs,
                    const uint32_t* __restrict__ step, uint64_t limit_ns) {
   pdl_wait();
+  after_wait(windows, step);
   if (!peer_barrier(windows, rank, world, 0, step[0] + 1, limit_ns)) return;   // nothing is pulled
   int64_t per = 0;
   for (int s = 0; s < segs.n; ++s) per += segs.units[s];
@@ -128,6 +130,7 @@ combine_push_kernel(const float* __restrict__ y, const float* __restrict__ wts, 
   const int r = blockIdx.x;
   const int d = (blockIdx.y * 256 + threadIdx.x) * 4;
   pdl_wait();
+  after_wait(y, wts, pick, windows, step);
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) step[0] += 1;     // read by the kernels before and after only
   if (step_failed()) return;                          // a barrier of this step ran out: store nothing into the peers
   if (d < D) {
@@ -156,6 +159,7 @@ peer_push_kernel(const float4* __restrict__ partial, uint8_t* const* __restrict_
                  int rows, int D, uint32_t* __restrict__ step) {
   const int r = blockIdx.x;
   pdl_wait();
+  after_wait(partial, windows, step);
   if (blockIdx.x == 0 && threadIdx.x == 0) step[0] += 1;
   if (step_failed()) return;                          // a barrier of this step ran out: store nothing into the peers
   const int home = r / rows, j = r - home * rows;
@@ -170,6 +174,7 @@ __global__ void __launch_bounds__(256)
 window_picks_kernel(const int* __restrict__ pick, const float* __restrict__ wts, int lo, int n,
                     int* __restrict__ pick_out, float* __restrict__ wts_out, int count) {
   pdl_wait();
+  after_wait(pick, wts);
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i < count) {
     const int e = pick[i] - lo;
@@ -190,6 +195,7 @@ peer_sum_kernel(uint8_t* const* __restrict__ windows, int rank, int64_t p_offset
                 int extra_w_stride, const __nv_bfloat16* __restrict__ residual, const uint32_t* __restrict__ step,
                 uint64_t limit_ns) {
   pdl_wait();
+  after_wait(windows, extra, extra_w, residual, step);
   if (step_failed()) return;                          // the tokens barrier ran out: out keeps what it held
   if (!peer_barrier(windows, rank, world, 1, step[0], limit_ns)) return;
   const float* part = reinterpret_cast<const float*>(windows[rank] + p_offset);

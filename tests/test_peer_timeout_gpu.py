@@ -104,3 +104,34 @@ def test_a_complete_table_passes_and_the_limit_is_checked(short_limit):
     assert _lib.kernel_status() == 0 and int(dst.min()) == 7
     with pytest.raises(ValueError):
         _lib.set_wait_limit_ms(0)
+
+
+def test_steps_in_a_row_each_follow_their_own_rows(pdl):
+    """One rank, eight steps enqueued without a pause, every kernel right behind the one whose results it reads: picks,
+    weights, rows, the step count and the residual are this step's.  Exact: whole numbers that bf16 and fp32 hold."""
+
+    from tensorfold_b200 import _lib
+
+    rows, slots, dims, n = 48, 2, 512, 4
+    win, table, _, _, p_off = _window(1, rows, dims)
+    step = torch.zeros(1, dtype=torch.int32, device=DEV)
+    st = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device=DEV).manual_seed(3)
+
+    def whole(shape, top, dtype):
+        return torch.randint(0, top, shape, generator=g, device=DEV).to(dtype)
+
+    steps = [(whole((rows, slots), 2 * n, torch.int32), whole((rows, slots), 5, torch.float32),
+              whole((rows, slots, dims), 9, torch.float32), whole((rows, dims), 17, torch.bfloat16)) for _ in range(8)]
+    pick, wts = torch.zeros((rows, slots), dtype=torch.int32, device=DEV), torch.zeros((rows, slots), device=DEV)
+    outs = [torch.zeros((rows, dims), device=DEV) for _ in steps]
+    for (p, w, y, h), out in zip(steps, outs):
+        _lib.call("tfb_window_picks", p.data_ptr(), w.data_ptr(), 0, n, pick.data_ptr(), wts.data_ptr(), rows * slots, st)
+        _lib.call("tfb_combine_push", y.data_ptr(), wts.data_ptr(), pick.data_ptr(), 0, n, table.data_ptr(), p_off, 0, rows,
+                  rows, slots, dims, step.data_ptr(), st)
+        _lib.call("tfb_peer_sum", table.data_ptr(), 0, p_off, 1, rows, dims, out.data_ptr(), 1, 0, 0, 1, h.data_ptr(),
+                  step.data_ptr(), st)
+    torch.cuda.synchronize()
+    assert _lib.kernel_status() == 0 and int(step) == len(steps)
+    for (p, w, y, h), out in zip(steps, outs):
+        assert torch.equal(out, ((w * (p < n)).unsqueeze(-1) * y).sum(1) + h.float())

@@ -12,8 +12,11 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "tensorfold_b200" / "csrc"
-FILES = ["exl3.cu", "pack.cu", "routing.cu"]
-VOLATILE_READS = {"router_kernel": {"W"}, "router_rows_kernel": {"W"}, "router_mma_kernel": {"W"}, "route_kernel": {"W"}}
+FILES = ["exl3.cu", "experts_decode.cu", "experts_prefill.cu", "pack.cu", "peer.cu", "routing.cu"]
+VOLATILE_READS = {"router_kernel": {"W"}, "router_rows_kernel": {"W"}, "router_mma_kernel": {"W"}, "route_kernel": {"W"},
+                  "decode_kernel": {"W"}, "prefill_kernel": {"W"}}
+# read and counted up by one kernel of a step, read by the next
+COUNTERS = {"combine_push_kernel": {"step"}, "peer_push_kernel": {"step"}}
 # addresses that hang on a value read behind the wait: the input scales of the pair's expert
 DEPENDENT_ADDRESSES = {"exl3_prologue_kernel": {"suh0", "suh1"}}
 
@@ -42,6 +45,7 @@ def untied(name: str, params: str, body: str) -> set[str]:
     if "pdl_wait()" not in body:
         return set()
     invariant = {p.split()[-1].lstrip("*&") for p in params.split(",") if "__restrict__" in p and "const" in p}
+    invariant |= COUNTERS.get(name, set())
     tied = {n.strip() for call in re.findall(r"after_wait\(([^)]*)\)", body) for n in call.split(",")}
     return invariant - tied - VOLATILE_READS.get(name, set()) - DEPENDENT_ADDRESSES.get(name, set())
 
