@@ -762,9 +762,9 @@ grouped_tc_kernel(const GroupedArgs a) {
     const uint8_t* src = T + (size_t)lane * row_stride + (size_t)blk * row_bytes;
     const int c = lane & 7, r0 = lane >> 3;
     const __half* xk = xin + c * 8;
-    uint32_t row[PER];                                // in 8 inputs
+    uint32_t row[PER];                                // in 128 inputs (K is a multiple): 32 bits hold 2^39 inputs
 #pragma unroll
-    for (int j = 0; j < PER; ++j) row[j] = (uint32_t)max(pair_sh[r0 + 4 * j], 0) * (uint32_t)(a.K >> 3);
+    for (int j = 0; j < PER; ++j) row[j] = (uint32_t)max(pair_sh[r0 + 4 * j], 0) * (uint32_t)(a.K >> 7);
     int s = 0, ph = 1, back = 0, sp = 0, pph = 1;     // ph, pph: a ring's first round finds every stage free
     constexpr int rows = 2 * TC_STEP / 16;            // K is a multiple of 128: whole stages
     int p = 0;
@@ -791,7 +791,7 @@ grouped_tc_kernel(const GroupedArgs a) {
         const int r = r0 + 4 * j;
         if (r < cnt) {
           uint8_t* dst = btile + 4 * j * 128 + ((c ^ (r & 7)) << 4);
-          const __half* from = xk + (size_t)row[j] * 8;
+          const __half* from = xk + (size_t)row[j] * 128;
           cp_async16(dst, from);
           cp_async16(dst + SM::B_TILE, from + TC_STEP);
         }

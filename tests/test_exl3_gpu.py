@@ -396,3 +396,41 @@ def test_prompt_matmul_into_unaligned_rows(rows, dtype):
     wide = torch.full((rows, 387), 7.0, dtype=dtype, device=DEV)
     prefill.matmul(layer, x, wide[:, 1:385], ws)
     assert torch.equal(wide[:, 1:385], want) and (wide[:, 0] == 7.0).all() and (wide[:, 385:] == 7.0).all()
+
+
+def test_wide_items_reach_inputs_past_2_to_the_35():
+    """Rotated inputs of more than 2^35 values (68 GB): the wide items' rows at the far end are those the narrow items read,
+    not the ones 2^35 values before them (which hold zeros)."""
+
+    from tensorfold_b200 import _lib
+
+    K, N, bits, count = 1 << 17, 128, 4, 32
+    first = (1 << 35) // K
+    P = first + count
+    if torch.cuda.mem_get_info()[0] < P * K * 2 + (4 << 30):
+        pytest.skip("needs 73 GB of free device memory")
+    g = torch.Generator().manual_seed(6)
+    t = _trellis(K, N, 2 * bits, g)
+    svh = _scale(N, 1.0, g)
+    x = torch.empty((P, K), dtype=torch.float16, device=DEV)
+    x[:count].zero_()
+    x[first:] = torch.randn((count, K), generator=g).half().to(DEV)
+
+    def ints(v):
+        return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    tp, k2 = torch.tensor([t.data_ptr()], dtype=torch.int64, device=DEV), ints([2 * bits])
+    members, arrive, z = ints(list(range(first, P))), ints([0, 0]), torch.zeros((P, N), device=DEV)
+    got = {}
+    for per in (16, 32):
+        items = ints([[0, at, per] for at in range(0, count, per)])
+        counts, y = ints([count // per, 1]), torch.zeros((P, N), device=DEV)
+        _lib.call("tfb_exl3_down", x.data_ptr(), tp.data_ptr(), k2.data_ptr(), items.data_ptr(), counts.data_ptr(),
+                  members.data_ptr(), z.data_ptr(), arrive.data_ptr(), svh.data_ptr(), y.data_ptr(), K, N, P, 0,
+                  count // per, 0, per, 0, 4, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert _lib.kernel_status() == 0
+        got[per] = y[first:].clone()
+    del x
+    torch.cuda.empty_cache()
+    assert float(got[16].abs().min()) > 0 and torch.equal(got[16], got[32])
