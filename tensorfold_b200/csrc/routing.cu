@@ -715,8 +715,11 @@ route_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, const __nv_b
 // Combine: out[r, d] = sum over slots in slot order of wts[r, s] * y[r, s, d] (fp32 fma chain from 0), rounded once.
 // (src/tensorfold/cuda/moe.py:131-151; src/tensorfold/cuda/exl3/experts.cu:181-190 for the fp32-out form.)
 // ================================================================================================================
-// With `pick`: only slots whose expert id lies in [lo, lo + n) take part (the others' rows are not read).
-template <typename TY, typename TO>
+// WINDOW: only slots whose expert id pick[r, s] lies in [lo, lo + n) take part (the others' rows are not read).  Bound by
+// latency at a few rows and by HBM at many.  The plain form has the rows of four slots in flight (8 slots of 2048 columns: 1
+// row 1.6 us, 64 rows 1.9, 2048 rows 22.4; left to the compiler 1.8, 2.0, 24.1; eight slots 1.7, 1.8, 24.7); the window, which
+// skips most slots, takes them one by one (2048 rows, half of the slots: 13.8 us; four at a time 15.2).
+template <typename TY, typename TO, bool WINDOW>
 __global__ void __launch_bounds__(256)
 combine_kernel(const TY* __restrict__ y, const float* __restrict__ wts, TO* __restrict__ out, int S, int D,
                const int* __restrict__ pick, int lo, int n) {
@@ -724,16 +727,11 @@ combine_kernel(const TY* __restrict__ y, const float* __restrict__ wts, TO* __re
   const int d = (blockIdx.y * 256 + threadIdx.x) * 4;
   if (d >= D) return;
   pdl_wait();
-  after_wait(y, wts, pick);
+  after_wait(y, wts);
+  if constexpr (WINDOW) after_wait(pick);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int s = 0; s < S; ++s) {
-    if (pick != nullptr) {
-      const int e = pick[(size_t)r * S + s] - lo;
-      if (e < 0 || e >= n) continue;
-    }
-    const float w = wts[(size_t)r * S + s];
+  auto load = [&](int s, float (&v)[4]) {
     const TY* src = y + ((size_t)r * S + s) * D + d;
-    float v[4];
     if constexpr (sizeof(TY) == 4) {
       const float4 f = *reinterpret_cast<const float4*>(src);
       v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
@@ -741,8 +739,34 @@ combine_kernel(const TY* __restrict__ y, const float* __restrict__ wts, TO* __re
       const uint2 u = *reinterpret_cast<const uint2*>(src);
       v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
     }
+  };
+  if constexpr (WINDOW) {
+    for (int s = 0; s < S; ++s) {
+      const int e = pick[(size_t)r * S + s] - lo;
+      if (e < 0 || e >= n) continue;
+      const float w = wts[(size_t)r * S + s];
+      float v[4];
+      load(s, v);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = fmaf(w, v[j], acc[j]);
+      for (int j = 0; j < 4; ++j) acc[j] = fmaf(w, v[j], acc[j]);
+    }
+  } else {
+    constexpr int B = 4;
+    for (int s0 = 0; s0 < S; s0 += B) {
+      float w[B], v[B][4];
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+        if (s0 + i < S) {
+          w[i] = wts[(size_t)r * S + s0 + i];
+          load(s0 + i, v[i]);
+        }
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+        if (s0 + i < S) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[j] = fmaf(w[i], v[i][j], acc[j]);
+        }
+    }
   }
   pdl_launch_dependents();
   TO* dst = out + (size_t)r * D + d;
@@ -1115,28 +1139,22 @@ extern "C" int tfb_route(const void* x, int64_t x_stride, const void* rows, floa
 #undef TFB_ROUTE
 }
 
+template <typename TY, typename TO>
+static cudaError_t combine_typed(const void* y, const float* wts, void* out, int T, int slots, int D, const int32_t* pick,
+                                 int lo, int n, cudaStream_t st) {
+  return launch(pick ? combine_kernel<TY, TO, true> : combine_kernel<TY, TO, false>, dim3(T, (D + 1023) / 1024), dim3(256), 0,
+                st, static_cast<const TY*>(y), wts, static_cast<TO*>(out), slots, D, pick, lo, n);
+}
+
 static int combine_launch(const void* y, int y_bf16, const float* wts, void* out, int out_f32, int T, int slots, int D,
                           const int32_t* pick, int lo, int n, void* stream) {
   TFB_REQUIRE(y && wts && out, "combine: null pointer");
   TFB_REQUIRE(D > 0 && D % 4 == 0 && slots >= 1, "combine: D must be a multiple of 4 and slots >= 1");
   TFB_REQUIRE(aligned16(y) && aligned16(out), "combine: y and out must be 16-byte aligned");
   if (T <= 0) return TFB_OK;
-  const dim3 grid(T, (D + 1023) / 1024);
-  auto st = static_cast<cudaStream_t>(stream);
-  cudaError_t e;
-  if (y_bf16 && out_f32)
-    e = launch(combine_kernel<__nv_bfloat16, float>, grid, dim3(256), 0, st, static_cast<const __nv_bfloat16*>(y), wts,
-               static_cast<float*>(out), slots, D, pick, lo, n);
-  else if (y_bf16)
-    e = launch(combine_kernel<__nv_bfloat16, __nv_bfloat16>, grid, dim3(256), 0, st,
-               static_cast<const __nv_bfloat16*>(y), wts, static_cast<__nv_bfloat16*>(out), slots, D, pick, lo, n);
-  else if (out_f32)
-    e = launch(combine_kernel<float, float>, grid, dim3(256), 0, st, static_cast<const float*>(y), wts,
-               static_cast<float*>(out), slots, D, pick, lo, n);
-  else
-    e = launch(combine_kernel<float, __nv_bfloat16>, grid, dim3(256), 0, st, static_cast<const float*>(y), wts,
-               static_cast<__nv_bfloat16*>(out), slots, D, pick, lo, n);
-  return check_cuda(e, "combine");
+  auto* typed = y_bf16 ? (out_f32 ? combine_typed<__nv_bfloat16, float> : combine_typed<__nv_bfloat16, __nv_bfloat16>)
+                       : (out_f32 ? combine_typed<float, float> : combine_typed<float, __nv_bfloat16>);
+  return check_cuda(typed(y, wts, out, T, slots, D, pick, lo, n, static_cast<cudaStream_t>(stream)), "combine");
 }
 
 extern "C" int tfb_combine(const void* y, int y_bf16, const float* wts, void* out, int out_f32, int T, int slots,

@@ -315,3 +315,25 @@ def test_add_moe_norm_against_float64(rows, d, slots, top_k, ydtype):
     assert float((out.double() - want_out).abs().max()) <= 2.0 ** -7 * float(want_out.abs().max())
     sums = out.float().view(rows, d // 64, 64).sum(2)
     assert torch.allclose(xs, sums, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("slots", [1, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_combine_over_any_number_of_slots(slots, dtype):
+    """The weighted sum with the slots' rows in flight four at a time, around multiples of four: exact on whole numbers,
+    and on others the bits of the window form, which adds the same slots one by one."""
+
+    from tensorfold_b200 import _lib, moe
+
+    rows, dims = 5, 1036
+    g = torch.Generator(device=DEV).manual_seed(slots)
+    whole = torch.randint(-9, 10, (rows, slots, dims), generator=g, device=DEV).to(dtype)
+    wts = torch.randint(1, 5, (rows, slots), generator=g, device=DEV).float()
+    got = moe.combine(whole, wts, torch.empty((rows, dims), device=DEV))
+    assert torch.equal(got, (wts.unsqueeze(-1) * whole.float()).sum(1))
+    y, wts = torch.randn((rows, slots, dims), generator=g, device=DEV).to(dtype), torch.rand((rows, slots), generator=g, device=DEV)
+    pick = torch.zeros((rows, slots), dtype=torch.int32, device=DEV)
+    window = torch.empty((rows, dims), device=DEV)
+    _lib.call("tfb_combine_window", y.data_ptr(), int(dtype == torch.bfloat16), wts.data_ptr(), pick.data_ptr(), 0, 1,
+              window.data_ptr(), 1, rows, slots, dims, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(moe.combine(y, wts, torch.empty_like(window)), window)
