@@ -192,6 +192,35 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
   return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity));
 }
 
+// The same without a call: one block of a dozen instructions.  A call, even one that is hardly ever made, binds the
+// registers that live across it; in a loop that holds many (16 pairs a warp) and that few warps run, that shows.  Where
+// the loops are short or walked by many warps the smaller code of the call is as good or better, so each loop uses what
+// it measured faster with: dense 4-bit, 16 to 64 rows (1024 x 1024) 8.8 us with the call, 8.5 inline; a dense EXL3 layer of
+// 6144 x 1024 at 3 bits, 16 rows, 60 and 53-55 us; one of 4.00 bits in 128 experts, 64 rows, 188 and 194 us.
+__device__ __forceinline__ bool mbar_wait_warp_inline(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p, q;\n.reg .u64 start, now;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+      "@p bra DONE;\n"
+      "mov.u64 start, %globaltimer;\n"
+      "AGAIN:\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+      "@p bra DONE;\n"
+      "mov.u64 now, %globaltimer;\n"
+      "sub.u64 now, now, start;\n"
+      "setp.lt.u64 q, now, 1000000000;\n"           // gives up after a second, as mbar_wait does
+      "@q bra AGAIN;\n"
+      "DONE:\n"
+      "selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_addr(bar)), "r"(parity), "r"(MBAR_NAP_NS)
+      : "memory");
+  const bool all = __all_sync(0xffffffffu, ok != 0);
+  if (!all) atomicCAS(&g_kernel_status, 0, ST_WAIT_TIMEOUT);
+  return all;
+}
+
 // global -> shared bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned), completion on `bar`
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(

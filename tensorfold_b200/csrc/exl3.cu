@@ -189,7 +189,7 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
 // four, whose inputs are loaded before the block's tiles are decoded.  x[pt]: the lane's pair (B column lane / 4 of
 // tile pt) at input 16 kt0 + 2 (lane % 4).  NPT: the mma tiles of eight pairs that are live (one decode feeds them all).
 // Returns false when a copy never landed.
-template <int CB, int K2, int PT, int NPT, int NTB, bool COMPACT>
+template <int CB, int K2, int PT, int NPT, int NTB, bool COMPACT, bool INLINE_WAIT>
 __device__ __forceinline__ bool warp_rows(const uint8_t* __restrict__ T, int ntiles, int kt0, int nkt, int nt0,
                                           const __half* const (&x)[PT], uint8_t* ring, uint64_t* bars, int lane,
                                           float (&acc)[NTB][PT][4]) {
@@ -247,7 +247,7 @@ __device__ __forceinline__ bool warp_rows(const uint8_t* __restrict__ T, int nti
               b[r][pt][1] = *reinterpret_cast<const uint32_t*>(xp[pt] + (r0 + r) * 16 + 8);
             }
           }
-        if (r0 == 0 && !mbar_wait_warp(bars + stage, phase)) {
+        if (r0 == 0 && !(INLINE_WAIT ? mbar_wait_warp_inline(bars + stage, phase) : mbar_wait_warp(bars + stage, phase))) {
           for (int g = f + 1; g < nslot && g < f + GR_STAGES; ++g)    // give the other copies in flight a while to land
             mbar_wait_for(bars + g % GR_STAGES, (g / GR_STAGES) & 1, 10000000ull);
           return false;
@@ -580,9 +580,13 @@ grouped_kernel(const GroupedArgs a) {
   bool ok = true;
   uint8_t* my_ring = ring + warp * (GR_STAGES * GR_SLOT_BYTES);
   uint64_t* my_bars = bars + warp * GR_STAGES;
-#define TFB_K2_BODY(K2_)                                                                                              \
-    ok = live > 1 ? warp_rows<CB, K2_, PT, PT, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc) \
-                  : warp_rows<CB, K2_, PT, 1, NTB, COMPACT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring, my_bars, lane, acc);
+  // (the build for 4.00 bits alone and the one with short loops are no faster with the wait inline)
+  constexpr bool INLINE_WAIT = K2F == 0 && !COMPACT;
+#define TFB_K2_BODY(K2_)                                                                                         \
+    ok = live > 1 ? warp_rows<CB, K2_, PT, PT, NTB, COMPACT, INLINE_WAIT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring,  \
+                                                                          my_bars, lane, acc)                     \
+                  : warp_rows<CB, K2_, PT, 1, NTB, COMPACT, INLINE_WAIT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring,   \
+                                                                         my_bars, lane, acc);
 #define TFB_K2(K2_) \
   case K2_:         \
     TFB_K2_BODY(K2_) \

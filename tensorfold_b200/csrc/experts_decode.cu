@@ -168,7 +168,8 @@ decode_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots, 
 #pragma unroll
       for (int ks = 1; ks < 4; ++ks) mma_bf16(xs[pt], ONES, ONES, ONES, ONES, xb[pt][2 * ks], xb[pt][2 * ks + 1]);
     }
-    if (gi == 0 && !mbar_wait_warp(bars + s, (fill / STAGES) & 1)) {
+    const uint32_t round = (fill / STAGES) & 1;
+    if (gi == 0 && !(PT == 2 ? mbar_wait_warp_inline(bars + s, round) : mbar_wait_warp(bars + s, round))) {
       // the copy never landed (recorded in the status word): give the other copies this warp issued a short while to
       // land, then the whole CTA leaves without storing anything
       for (int f = fill + 1; f < nslot && f < fill + STAGES; ++f) mbar_wait_for(bars + f % STAGES, (f / STAGES) & 1, 10000000ull);
