@@ -208,3 +208,20 @@ def test_item_bound_holds_for_every_split_of_the_pairs():
         assert made <= experts.max_items(p, e, tile) <= min(p, e) + p // tile
         assert sum((c + 15) // 16 for c in counts) <= x3.max_items(p, e)
     assert experts.max_items(17, 1, 8) == 3 and experts.max_items(16, 1, 8) == 2 and experts.max_items(0, 5, 8) == 0
+
+
+def test_hot_item_bound_holds_for_every_split_of_the_pairs():
+    """``max_big_items`` (what sizes the prompt kernel's launches of a split plan): never below the items of the experts
+    with ``hot`` pairs or more, never above the bound that takes every expert for hot."""
+
+    from tensorfold_b200 import experts
+
+    rng = np.random.default_rng(4)
+    for _ in range(3000):
+        e, hot = int(rng.integers(1, 40)), int(rng.integers(1, 300))
+        counts = np.floor(rng.pareto(0.7, e) * rng.integers(1, 60)).astype(int).clip(0, 2000)
+        pairs = int(counts.sum()) + int(rng.integers(0, 5))            # some picks may be no expert of the plan
+        made = sum((c + experts.PREFILL_TILE - 1) // experts.PREFILL_TILE for c in counts.tolist() if c >= hot)
+        assert made <= experts.max_big_items(pairs, e, hot) <= experts.max_items(pairs, e, experts.PREFILL_TILE)
+    assert experts.max_big_items(256, 128, 32) == 9 and experts.max_big_items(31, 128, 32) == 0
+    assert experts.max_big_items(64, 128, 32) == 2
