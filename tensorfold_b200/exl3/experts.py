@@ -26,12 +26,19 @@ K2_SUPPORTED = tuple(range(2, 17))   # half-bits a value: 1..8 bits and every ha
 LAUNCHES_PER_CALL = 4             # kernels one ``routed`` call with weights enqueues (3 without)
 ITEM_PAIRS = 16                   # pairs an item of the sort holds: two mma tiles share one decoded weight tile
 WIDE_ITEM_PAIRS = 32              # the same for the kernel's tensor-memory form, for calls with many pairs an expert
-# Pairs an expert on average from which a call sorts into the wide items (either way the same bits; whole calls measured,
-# narrow against wide items): widths 5 bits 12 pairs 292 / 292 us, 14 pairs 322 / 300; 3 bits 12 pairs 157 / 164, 16 pairs
-# 195 / 171.  At 4.00 bits the narrow items have a kernel build of their own: 14 pairs 274 / 303.  Where the widths differ
-# the narrow items run the build with short loops: 4.8 pairs 992 / 1002, 6.4 pairs 1023 / 1013, 11 pairs 1181 / 1061 - in a
-# launch of several waves (below that: not measured, the one-width line).
-WIDE_FROM, WIDE_FROM_FOUR, WIDE_FROM_MIXED = 14, 16, 6
+# Pairs an expert on average from which a call sorts into the wide items (either way the same bits).  Whole calls, narrow
+# against wide items in us, 128 experts of 2048 x 768 and 160 of 4096 x 1536:
+#   one width, 3 bits  10 pairs 273 / 273, 1086 / 1025; 12 288 / 279, 1149 / 1042; 14 322 / 286, 1280 / 1060
+#   5 bits             10 pairs 264 / 276, 1059 / 1019; 12 285 / 281, 1150 / 1037; 14 314 / 288, 1277 / 1054
+#   4.00 bits          12 pairs 241 / 282, 964 / 1042;  14 267 / 288, 1070 / 1059; 16 302 / 294, 1225 / 1079
+# Where the widths differ the line hangs on the inputs a block walks: its start and its empty pipeline cost the same
+# whatever they are.  128 experts of 1024 x 1536: 6 pairs 254 / 287, 11 287 / 301, 13 315 / 306; of 1024 x 640: 11 152 / 155, 13
+# 166 / 159; of 2048 x 768: 6 259 / 273, 7 274 / 277, 8 280 / 279; 64 of 2048 x 1536: 6 252 / 254, 7 263 / 256; 64 of 4096 x
+# 1280: 5 363 / 371, 6 386 / 373; 160 of 4096 x 1536: 5 977 / 985, 6 998 / 997, 8 1049 / 1013.  A launch of less than four
+# waves follows the one-width line, which is late for it (20 of 4096 x 1536: 4 pairs 170 / 162, 8 190 / 165; 32 of 1024 x
+# 512: 4 pairs 46 / 40, 8 56 / 41).
+WIDE_FROM, WIDE_FROM_FOUR = 14, 16
+WIDE_FROM_MIXED = ((4096, 6), (2048, 7), (0, 13))    # (inputs of gate and up from which, pairs an expert)
 
 # (16-column tiles a block, K-slice warps, K splits across blocks, tiles in flight): this library's one setting.
 # The split is by shape only; partial sums meet in warp order inside the block, so there is one split.
@@ -173,7 +180,7 @@ def wide_from(ex: "Exl3RoutedExperts", pairs: int) -> float:
     """The line for ``item_pairs`` of a layer."""
 
     if ex.mixed and min(pairs, ex.count) * (ex.width // 128) * 2 >= WIDE_WAVES_BLOCKS:
-        return WIDE_FROM_MIXED
+        return next(line for dims, line in WIDE_FROM_MIXED if ex.dims >= dims)
     return WIDE_FROM_FOUR if ex.k2_gu == ex.k2_d == (8, 8) else WIDE_FROM
 
 
