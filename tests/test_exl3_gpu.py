@@ -308,25 +308,38 @@ def test_blocks_of_two_or_four_column_tiles_give_the_same_bits(R, monkeypatch):
     assert bool(torch.isfinite(outs[0][0]).all()) and float(outs[0][0].abs().max()) > 0
 
 
+@pytest.mark.parametrize("cb", [0, 1, 2])
 @pytest.mark.parametrize("R", [1, 37, 200])
-def test_the_short_loop_build_for_mixed_widths_gives_the_same_bits(R, monkeypatch):
+def test_the_short_loop_build_for_mixed_widths_gives_the_same_bits(R, cb, monkeypatch):
     """A projection whose tensors differ in width runs the kernel's build with short loops (blocks of different widths
-    then share an SM's instruction cache); the all-widths build with unrolled loops gives the same bits."""
+    then share an SM's instruction cache) in a large launch; here it is asked for in a small one.  Every width of the
+    format, items of 16 pairs: the bits of the all-widths build with unrolled loops."""
 
+    from tensorfold_b200 import _lib
     from tensorfold_b200.exl3 import experts
 
-    E, D, I, TOPK = 12, 256, 384, 3
-    ex, _ = _layer(E, D, I, [((2, 16, 7)[e % 3], (5, 3, 8)[e % 3], (4, 9, 12, 6)[e % 4]) for e in range(E)], 0, 33)
-    assert ex.mixed
-    g = torch.Generator().manual_seed(15)
+    E, D, I, TOPK = 15, 256, 384, 3
+    ex, _ = _layer(E, D, I, [(2 + e, 16 - e, 2 + (e + 5) % 15) for e in range(E)], cb, 35)
+    g = torch.Generator().manual_seed(16)
     x = torch.randn((R, D), generator=g).to(torch.bfloat16).to(DEV)
     sel, w = _picks(E, R, TOPK, g)
+    monkeypatch.setattr(experts, "CROWDED_BLOCKS", 0)
+    monkeypatch.setattr(experts, "item_pairs", lambda *shape: experts.ITEM_PAIRS)
+    call, seen = _lib.call, []
+
+    def spy(name, *args):
+        if name in ("tfb_exl3_gateup", "tfb_exl3_down"):
+            seen.append(args[-3])                       # k2_all
+        call(name, *args)
+
+    monkeypatch.setattr(_lib, "call", spy)
     outs = []
     for compact in (True, False):
         monkeypatch.setattr(experts, "COMPACT_MIXED", compact)
         s = experts.Scratch(ex, R, TOPK)
         outs.append((experts.routed(x, sel, w, ex, s, None, R).clone(), s.y[:R * TOPK].clone()))
     torch.cuda.synchronize()
+    assert seen == [-1, -1, 0, 0] and _lib.kernel_status() == 0
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     assert bool(torch.isfinite(outs[0][0]).all()) and float(outs[0][0].abs().max()) > 0
 

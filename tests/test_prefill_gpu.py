@@ -129,11 +129,13 @@ def test_prefill_layer_against_the_oracle(shared, pdl):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("rows", [1, 15, 16, 17, 191, 192, 193])
+@pytest.mark.parametrize("tile", [64, 192])
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 63, 64, 65, 191, 192, 193])
 @pytest.mark.parametrize("width, dims", [(32, 64), (96, 128), (160, 192)])
-def test_tile_edges_equal_the_rounded_weights_product(rows, width, dims, dtype):
+def test_tile_edges_equal_the_rounded_weights_product(rows, width, dims, tile, dtype):
     """Items around the MMA's row granularity and capacity, column counts that leave a unit's blocks missing (one matrix:
-    128 columns a unit, gate and up: 64) and one to three groups of inputs, one expert.  Bounds: the gate/up output is
+    128 columns a unit, gate and up: 64) and one to three groups of inputs, one expert, in the build for items of up to 64
+    pairs and in the one for 192.  Bounds: the gate/up output is
     within two bf16 roundings (2^-7) of the rounded reference's largest value, the fp32 down product within the error of a
     K <= 192 fp32 sum (1e-5 of the largest value)."""
 
@@ -143,7 +145,7 @@ def test_tile_edges_equal_the_rounded_weights_product(rows, width, dims, dtype):
     ex = experts.make([gate, up], mlx(1, dims, 64, 7, dtype), 64)  # (the down projection is not run)
     x = (torch.randn((rows, dims), generator=torch.Generator().manual_seed(rows)) * 0.5).to(torch.bfloat16).to(DEV)
     plan = experts.Plan(rows, 1, 1, DEV, prefill=True)
-    experts.route(torch.zeros((rows, 1), dtype=torch.int32, device=DEV), plan)
+    experts.route(torch.zeros((rows, 1), dtype=torch.int32, device=DEV), plan, tile)
     act = torch.full((rows, width), float("nan"), dtype=torch.bfloat16, device=DEV)
     experts.gate_up(x, ex, plan, act, rows)
     torch.cuda.synchronize()
