@@ -293,7 +293,7 @@ __device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_
 
 // Shared memory of a CTA: the trellis ring (stages of 128 inputs x 128 columns: 1024 K2 bytes), the B ring (32 pairs x
 // 128 inputs a stage, two 128-byte-swizzled tiles), the pair table, barriers.  After the main loop the trellis ring's
-// memory takes the accumulators ([32][128] fp32) and, in a cluster, the other parts'.
+// memory takes the sums ([32][128] fp32).
 struct TrellisSmem {
   static constexpr int RING_BYTES = 65536, SP_MAX = 8;
   static constexpr int B_TILE = TC_PAIRS * 128, SB = 4;
@@ -685,9 +685,13 @@ __device__ __forceinline__ uint32_t umma_idesc_f16(int n) {
 // 32 pairs and touches neither shared memory nor further registers).
 // The four parts of K are four accumulators, added in order: the sums of grouped_kernel's four warps, bit for bit.
 //
-// What bounds it: instruction issue in the decode, about 60 instructions a tile and lane with the pipeline's own.
+// What bounds it: latency in the decoding warps' pipeline, at about 60 instructions a tile and lane.  A B200 at 4.00 bits, 128
+// experts of 2048 x 768, 20 pairs an expert: the schedulers issue in 0.58 of the cycles (down 0.52), the ALU pipe is 0.48
+// (0.40) busy, the multiply pipe 0.41 (0.33), DRAM 0.16; of 13 cycles from one of a warp's instructions to the next, 8 wait for
+// a long-latency result, the pipeline's barriers among them (a set has one A stage and waits for it before it decodes).
 // Two CTAs of sixteen decoding warps fill an SM's tensor memory.
-// TC_MEASURED
+// The layer takes 310 us, with the register kernel 374; 160 experts of 4096 x 1536 with widths of 2 to 8 bits at 512 tokens
+// 1655 us with an mma.sync form, 1315 with this one.
 template <int CB>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 grouped_tc_kernel(const GroupedArgs a) {
@@ -1402,8 +1406,8 @@ static int exl3_grouped_launch(const char* who, exl3::GroupedArgs a, int cb, int
 // items / counts / members: the prologue's sort; z: fp32 scratch [2, P, N]; arrive: int scratch
 // [max_items * N / 128], zero before the first call (every call leaves it zero); max_items >= the sort's items.
 // sorted_g / sorted_u (or null): the prologue's width orders of the two matrices ([., 4] each).  item_pairs: 16 or 32,
-// the most pairs an item of the sort holds (32: one decode of a weight tile serves up to 32 pairs, at more registers
-// a thread - for calls with many pairs an expert); a pair's bits do not depend on it.  k2_all: 0, or the width that
+// the most pairs an item of the sort holds (32: the tensor-memory kernel, in which one decode of a weight tile serves up to
+// 32 pairs - for calls with many pairs an expert); a pair's bits do not depend on it.  k2_all: 0, or the width that
 // every k2_g and k2_u entry has (a promise: the launch may then use a kernel built for that width alone; a tensor of
 // another width sets the status word and stores nothing); -1: the widths differ (a build of the kernel with short
 // loops: blocks of different widths then share an SM's instruction cache).  col_tiles: 4 or 2, the 16-column tiles a block takes - 2

@@ -4,24 +4,26 @@
 // the WEIGHTS are the MMA's A operand (M = 128 rows: 128 output columns of one matrix, or 64 columns of gate and the
 // same 64 of up), the item's PAIRS the B operand (N = pairs rounded up to 16, <= 192), so an expert with 140 pairs
 // costs 144 / 128 of a full tile instead of two.  Per group of 64 inputs (one pipeline stage):
-//   warp 13 (a lane)   bulk-copies the packed blocks into a deep staging ring;
-//   warps 8-11         gather the pairs' input rows with 16-byte cp.async into the 128-byte-swizzled B tile;
-//   warps 0-7          turn nibbles into the prefill form's bf16 weights (w = bf16(q * s + b), one rounding) and
-//                      store them straight into TENSOR MEMORY, a weight row a lane (tcgen05.st): two sets of four
-//                      warps take the even and the odd stages, each set with an A stage of its own;
-//   warp 12 (a lane)   issues tcgen05.mma (cta_group::1, kind::f16, M = 128, K = 16; A from tensor memory, B from
-//                      shared memory) into fp32 accumulators in tensor memory, and commits each stage back.
-// After the last group warps 0-11 read the accumulators (tcgen05.ld), apply the epilogue and store rows by pair id.
+//   warps 0-7    turn nibbles into the prefill form's bf16 weights (w = bf16(q * s + b), one rounding) and store them
+//                straight into TENSOR MEMORY, a weight row a lane (tcgen05.st): two sets of four warps take the even and
+//                the odd stages, each set with an A stage of its own;
+//   gathering    warps (8-11, or 8-9 in the build for small items): the pairs' input rows with 16-byte cp.async into the
+//                128-byte-swizzled B tile;
+//   MMA          warp (the next): one lane issues tcgen05.mma (cta_group::1, kind::f16, M = 128, K = 16; A from tensor
+//                memory, B from shared memory) into fp32 accumulators in tensor memory, and commits each stage back;
+//   copying      warp (the last): bulk copies of the packed blocks into a deep staging ring, a lane a column block.
+// After the last group two or three warps a lane quarter read the accumulators (tcgen05.ld), apply the epilogue and store
+// rows by pair id.
 // One fp32 chain over K in group order: a pair's bits do not depend on its item, its chunk or the call.
 //
-// What bounds it: shared-memory bandwidth and tensor issue, about even.  With the A tiles in shared memory a stage of
-// gate/up moved 154 KB through it at 192 pairs (of it 64 KB A written and read) and the K loop ran at 0.91 us a stage;
-// without them and with two CTAs an SM (256 of the 512 tensor-memory columns each: 192 of accumulators, two A stages
-// of 32; under 113 KB of shared memory; three CTAs in the build for items of up to 64 pairs) one unit's start, epilogue
-// and waits run under the others' K loops.
-// A B200 at 2048 tokens of 128 experts (2048 x 768, top 8): gate/up 220 -> 158 us, down 182 -> 110 us; at 317 tokens with
-// a shared expert (20 pairs an expert, items of 64) 172 -> 93 and 143 -> 65 us.  What is left is instruction issue (two thirds of the slots, the ALU pipe
-// 60 % busy): about 1000 of the dequantising warps' instructions a stage against 256 cycles of MMA.
+// What bounds it: instruction issue of the dequantisation.  On a B200 at 2048 tokens of 128 experts (2048 x 768, top 8) the
+// schedulers issue in 0.74 of the cycles of gate/up (down 0.67), the ALU pipe is 0.59 (0.50) busy, the multiply pipe 0.47
+// (0.41), tcgen05 0.34 (0.25), shared memory 0.32, DRAM 0.19; about 1000 of the dequantising warps' instructions a stage
+// stand against 256 cycles of MMA.  The build for small items at 317 tokens with a shared expert: issue 0.73 (0.66), ALU
+// 0.60 (0.52), tcgen05 0.13 (0.10), and more warps that wait for their inputs.
+// With the A tiles in shared memory a stage of gate/up moved 154 KB through it at 192 pairs (of it 64 KB A written and
+// read) and one CTA filled an SM; without them two or three CTAs share it, and one unit's start, epilogue and waits run
+// under the others' K loops.  gate/up 220 -> 158 us, down 182 -> 110 us at 2048 tokens; 172 -> 93 and 143 -> 65 us at 317.
 // (Replaces src/tensorfold/cuda/experts_prefill.cu:31-195: prefill_kernel and its launch.)
 
 #include "api.h"
@@ -34,8 +36,8 @@ constexpr int PF_MAXP = 192;            // pairs an item may hold (MMA N)
 constexpr int PF_SMALL_MAXP = 64;       // the same in the build for plans of small items
 constexpr int PF_DQ_WARPS = 8;          // warps 0-7: dequantise (two sets of four), then the epilogue
 
-// What the two builds differ in.  Items of up to 192 pairs: two CTAs an SM.  Items of up to 64: half the accumulators and a
-// third of the B ring, two gathering warps - three CTAs, because a unit of few pairs is mostly start, latency and epilogue.
+// What the two builds differ in.  Items of up to 192 pairs: two CTAs an SM.  Items of up to 64: a third of the accumulators
+// and of the B ring, two gathering warps - three CTAs, because a unit of few pairs is mostly start, latency and epilogue.
 // (317 tokens, top 8 of 128 and a shared expert: gate/up 119 us in the large build, 93 in this one, down 84 and 65.)
 template <int MAXP>
 struct PrefillShape {
@@ -267,7 +269,7 @@ prefill_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, int slots,
     }
     __syncwarp();
   } else if (warp >= PF_DQ_WARPS) {
-    // ---------------- warps 8-11: gather the pairs' input rows into the swizzled B tiles ----------------
+    // ---------------- the gathering warps: the pairs' input rows into the swizzled B tiles ----------------
     // thread -> chunk c of rows r0, r0 + GA_ROWS, ...: the row pointers stay in registers for the whole K loop
     constexpr int GA_PER = MAXP / SH::GA_ROWS;       // 16-byte chunks a thread a stage
     const int gt = tid - PF_DQ_WARPS * 32, c = gt & 7, r0 = gt >> 3;
