@@ -526,7 +526,8 @@ enum GroupedEpilogue : int { GE_NONE = 0, GE_GATEUP = 1, GE_DOWN = 2 };
 // alone - a tenth of the code, which matters where a CTA's life is short (one token: the dominant stall of the
 // all-widths kernel was the instruction fetch).
 // NTB: 16-column tiles a CTA (4, or 2 where the launch would otherwise have too few CTAs to fill the GPU).
-template <int CB, int K2F, int NTB, bool COMPACT>
+// INLINE_WAIT: a slot's wait without a call, for launches that leave a scheduler one to three warps (exl3_grouped_launch).
+template <int CB, int K2F, int NTB, bool COMPACT, bool INLINE_WAIT>
 __global__ void __launch_bounds__(GR_WARPS * 32)
 grouped_kernel(const GroupedArgs a) {
   constexpr int PT = GR_PT, PAIRS = GR_PAIRS, GR_RED_STRIDE = NTB * 16 + 1;
@@ -580,8 +581,6 @@ grouped_kernel(const GroupedArgs a) {
   bool ok = true;
   uint8_t* my_ring = ring + warp * (GR_STAGES * GR_SLOT_BYTES);
   uint64_t* my_bars = bars + warp * GR_STAGES;
-  // (the build for 4.00 bits alone and the one with short loops are no faster with the wait inline)
-  constexpr bool INLINE_WAIT = K2F == 0 && !COMPACT;
 #define TFB_K2_BODY(K2_)                                                                                         \
     ok = live > 1 ? warp_rows<CB, K2_, PT, PT, NTB, COMPACT, INLINE_WAIT>(T, a.N >> 4, kt0, nkt, nt0, x, my_ring,  \
                                                                           my_bars, lane, acc)                     \
@@ -1382,12 +1381,22 @@ static int exl3_grouped_launch(const char* who, exl3::GroupedArgs a, int cb, int
   const dim3 block(exl3::GR_WARPS * 32);
   const bool four = k2_all == 8;                      // the one width with a kernel of its own (4.00 bits a weight)
   const bool narrow = col_tiles == exl3::GR_NARROW_NTB;
-#define TFB_GR4(CB_, K2F_, NTB_, COMPACT_) launch(exl3::grouped_kernel<CB_, K2F_, NTB_, COMPACT_>, grid, block, 0, st, a)
-#define TFB_GR(CB_)                                                  \
-  e = k2_all == -1 ? TFB_GR4(CB_, 0, exl3::GR_NTB, true)             \
-      : narrow     ? TFB_GR4(CB_, 8, exl3::GR_NARROW_NTB, false)     \
-      : four       ? TFB_GR4(CB_, 8, exl3::GR_NTB, false)            \
-                   : TFB_GR4(CB_, 0, exl3::GR_NTB, false)
+  // Few items with many pairs each: a warp mostly waits for its own chain and holds two live tiles of pairs, and the call
+  // behind a slot's wait costs it registers (one tensor of 6144 x 1024, 3 bits, 16 rows: 60.7 us with the call, 53.1 without;
+  // 20 experts of 4096 x 1536, 8 pairs each: 167.6 and 162.3).  Else the shorter code of the call is the faster (one row of
+  // 4096 x 4096: 33.5 and 34.7; 128 experts of 2048 x 768, 5 rows: 73.4 and 75.7, 64 rows: 210.7 and 214.8).  By what both
+  // launches of a layer share: with gate/up in one build and down in the other they miss the instruction cache (20 experts,
+  // 8 rows: 141.8 -> 150.7 us).  The build for 4.00 bits gains nothing either way.
+  constexpr int INLINE_WAIT_ITEMS = 64;
+  const bool few = max_items <= INLINE_WAIT_ITEMS && a.P > 4 * max_items;
+#define TFB_GR4(CB_, K2F_, NTB_, COMPACT_, INLINE_) \
+  launch(exl3::grouped_kernel<CB_, K2F_, NTB_, COMPACT_, INLINE_>, grid, block, 0, st, a)
+#define TFB_GR(CB_)                                                      \
+  e = k2_all == -1 ? TFB_GR4(CB_, 0, exl3::GR_NTB, true, false)          \
+      : narrow     ? TFB_GR4(CB_, 8, exl3::GR_NARROW_NTB, false, false)  \
+      : four       ? TFB_GR4(CB_, 8, exl3::GR_NTB, false, false)         \
+      : few        ? TFB_GR4(CB_, 0, exl3::GR_NTB, false, true)          \
+                   : TFB_GR4(CB_, 0, exl3::GR_NTB, false, false)
   if (cb == 0) {
     TFB_GR(0);
   } else if (cb == 1) {

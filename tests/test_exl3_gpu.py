@@ -447,3 +447,29 @@ def test_wide_items_reach_inputs_past_2_to_the_35():
     del x
     torch.cuda.empty_cache()
     assert float(got[16].abs().min()) > 0 and torch.equal(got[16], got[32])
+
+
+@pytest.mark.parametrize("cb, k2", [(0, 6), (1, 2), (2, 16), (0, 0), (2, 0)])
+@pytest.mark.parametrize("R", [1, 40])
+def test_small_and_large_launches_of_one_width_give_the_same_bits(R, cb, k2, monkeypatch):
+    """The register kernel's build for launches of few items against the one for many (the same call with room for more
+    items, whose blocks find none): one width, and widths that differ (k2 0); one row takes the latter both times."""
+
+    from tensorfold_b200 import _lib
+    from tensorfold_b200.exl3 import experts
+
+    E, D, I, TOPK = 8, 256, 384, 3
+    ex, _ = _layer(E, D, I, [((k2,) * 3 if k2 else (2 + e, 16 - e, 5 + e)) for e in range(E)], cb, 37)
+    g = torch.Generator().manual_seed(18)
+    x = torch.randn((R, D), generator=g).to(torch.bfloat16).to(DEV)
+    sel, w = _picks(E, R, TOPK, g)
+    monkeypatch.setattr(experts, "item_pairs", lambda *shape: experts.ITEM_PAIRS)
+    outs = []
+    for room in (None, 400):                                          # 400 items: 4800 blocks of gate/up, 1600 of down
+        if room:
+            monkeypatch.setattr(experts, "max_items", lambda *shape: room)
+        s = experts.Scratch(ex, R, TOPK)
+        outs.append(experts.routed(x, sel, w, ex, s, None, R).clone())
+    torch.cuda.synchronize()
+    assert _lib.kernel_status() == 0 and torch.equal(outs[0], outs[1])
+    assert bool(torch.isfinite(outs[0]).all()) and float(outs[0].abs().max()) > 0
