@@ -716,9 +716,11 @@ route_kernel(const __nv_bfloat16* __restrict__ X, int64_t x_stride, const __nv_b
 // (src/tensorfold/cuda/moe.py:131-151; src/tensorfold/cuda/exl3/experts.cu:181-190 for the fp32-out form.)
 // ================================================================================================================
 // WINDOW: only slots whose expert id pick[r, s] lies in [lo, lo + n) take part (the others' rows are not read).  Bound by
-// latency at a few rows and by HBM at many.  The plain form has the rows of four slots in flight (8 slots of 2048 columns: 1
-// row 1.6 us, 64 rows 1.9, 2048 rows 22.4; left to the compiler 1.8, 2.0, 24.1; eight slots 1.7, 1.8, 24.7); the window, which
-// skips most slots, takes them one by one (2048 rows, half of the slots: 13.8 us; four at a time 15.2).
+// latency at a few rows and by HBM at many.  The plain form has the rows of four slots in flight (8 slots of 2048 columns,
+// fp32: 1 row 1.6 us, 64 rows 1.9, 2048 rows 22.4; left to the compiler 1.8, 2.0, 24.1; eight slots 1.7, 1.8, 24.7).  bf16 rows
+// (2048: 13.4 us) take the slots past the last four one by one: predicates in every batch cost them 14.4, and fp32 rows are
+// the faster for them (512 rows 7.1 us and 7.5).  The window, which skips most slots, takes all of them one by one (2048 rows,
+// half of the slots: 13.8 us; four at a time 15.2).
 template <typename TY, typename TO, bool WINDOW>
 __global__ void __launch_bounds__(256)
 combine_kernel(const TY* __restrict__ y, const float* __restrict__ wts, TO* __restrict__ out, int S, int D,
@@ -740,33 +742,36 @@ combine_kernel(const TY* __restrict__ y, const float* __restrict__ wts, TO* __re
       v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
     }
   };
-  if constexpr (WINDOW) {
-    for (int s = 0; s < S; ++s) {
-      const int e = pick[(size_t)r * S + s] - lo;
-      if (e < 0 || e >= n) continue;
-      const float w = wts[(size_t)r * S + s];
-      float v[4];
-      load(s, v);
+  auto add = [&](float w, const float (&v)[4]) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[j] = fmaf(w, v[j], acc[j]);
-    }
-  } else {
+    for (int j = 0; j < 4; ++j) acc[j] = fmaf(w, v[j], acc[j]);
+  };
+  int s = 0;
+  if constexpr (!WINDOW) {
     constexpr int B = 4;
-    for (int s0 = 0; s0 < S; s0 += B) {
+    constexpr bool ALL = sizeof(TY) == 4;             // a last batch of fewer slots too, by predicates
+    for (; ALL ? s < S : s + B <= S; s += B) {
       float w[B], v[B][4];
 #pragma unroll
       for (int i = 0; i < B; ++i)
-        if (s0 + i < S) {
-          w[i] = wts[(size_t)r * S + s0 + i];
-          load(s0 + i, v[i]);
+        if (!ALL || s + i < S) {
+          w[i] = wts[(size_t)r * S + s + i];
+          load(s + i, v[i]);
         }
 #pragma unroll
       for (int i = 0; i < B; ++i)
-        if (s0 + i < S) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[j] = fmaf(w[i], v[i][j], acc[j]);
-        }
+        if (!ALL || s + i < S) add(w[i], v[i]);
     }
+  }
+  for (; s < S; ++s) {
+    if constexpr (WINDOW) {
+      const int e = pick[(size_t)r * S + s] - lo;
+      if (e < 0 || e >= n) continue;
+    }
+    const float w = wts[(size_t)r * S + s];
+    float v[4];
+    load(s, v);
+    add(w, v);
   }
   pdl_launch_dependents();
   TO* dst = out + (size_t)r * D + d;
